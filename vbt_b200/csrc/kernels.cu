@@ -580,37 +580,40 @@ __device__ __forceinline__ uint32_t pay_u32(const uint32_t* __restrict__ pw, uin
     return __funnelshift_r(ldw(pw, w), ldw(pw, w + 1u), (uint32_t)(b & 3u) * 8u);
 }
 
-// The basis row b_k(t) and the AC scales of a leaf with keep <= 7, read once for several controls.
-struct SciTerms {
-    float b[7], sc[6];
-    __device__ __forceinline__ SciTerms(const DeviceAsset& a, uint32_t t, int keep)
-    {
-        const float* brow = a.basis + (uint64_t)t * 64u;
-#pragma unroll
-        for (int k = 0; k < 7; ++k) b[k] = k < keep ? __ldg(brow + k) : 0.0f;
-#pragma unroll
-        for (int k = 0; k < 6; ++k) sc[k] = k + 1 < keep ? __ldg(a.scales + k) : 0.0f;
-    }
-};
-
-// sci_control for a control record at byte cb of at most 8 bytes (keep <= 7) that lies inside the
-// payload: the same products and compensated sum in the same order, the record read as two 32-bit
-// windows (DC half in bytes 0-1, AC byte k at byte k + 1).
-__device__ __forceinline__ float sci_control_fast(const uint32_t* __restrict__ pw, uint64_t cb, int keep,
-                                                  const SciTerms& tm)
+// A signed byte as a float without a conversion: 2^23 + (byte ^ 0x80) - (2^23 + 128), exact.
+__device__ __forceinline__ float byte_to_float(uint32_t word, uint32_t byte)
 {
-    const uint32_t w0 = pay_u32(pw, cb), w1 = keep > 3 ? pay_u32(pw, cb + 4u) : 0u;
+    const uint32_t m = __byte_perm(word ^ 0x80808080u, 0x4B000000u, 0x7650u | byte);
+    return __fsub_rn(__uint_as_float(m), 8388736.0f);
+}
+
+// sci_control for a record of at most 8 bytes (keep <= 7: DC half in bytes 0-1, AC byte k at byte
+// k + 1) at byte cb of the payload window `w`, inside the payload: the same products and compensated
+// sum in the same order, the record read as words and only the kept terms visited.
+__device__ __forceinline__ float sci_control_fast(const uint32_t* __restrict__ w, uint32_t cb, int keep,
+                                                  const float* __restrict__ brow, const float* __restrict__ scales)
+{
+    const uint32_t* p = w + (cb >> 2);
+    const uint32_t sh = (cb & 3u) * 8u;
+    const uint32_t x1 = __ldg(p + 1);
+    const uint32_t r0 = __funnelshift_r(__ldg(p), x1, sh);
+    const uint32_t r1 = keep > 2 ? __funnelshift_r(x1, __ldg(p + 2), sh) : 0u;
+    const float4 b03 = __ldg(reinterpret_cast<const float4*>(brow));   // rows of 64 floats
     float hi, lo;
-    two_prod(half_bits_to_float(w0 & 0xFFFFu), tm.b[0], hi, lo);
-#pragma unroll
-    for (int k = 1; k < 7; ++k) {
-        if (k < keep) {
-            const uint32_t byte = k + 1 < 4 ? (w0 >> (8 * (k + 1))) : (w1 >> (8 * (k - 3)));
-            const float coeff = __fmul_rn((float)(int8_t)(byte & 0xFFu), tm.sc[k - 1]);
-            float ph, pl;
-            two_prod(coeff, tm.b[k], ph, pl);
-            ff_add(hi, lo, ph, pl);
-        }
+    two_prod(half_to_float_exact(r0 & 0xFFFFu), b03.x, hi, lo);
+    auto term = [&](uint32_t word, uint32_t byte, int k, float b) {
+        float ph, pl;
+        two_prod(__fmul_rn(byte_to_float(word, byte), __ldg(scales + k - 1)), b, ph, pl);
+        ff_add(hi, lo, ph, pl);
+    };
+    if (keep > 1) term(r0, 2u, 1, b03.y);
+    if (keep > 2) term(r0, 3u, 2, b03.z);
+    if (keep > 3) term(r1, 0u, 3, b03.w);
+    if (keep > 4) {
+        const float4 b47 = __ldg(reinterpret_cast<const float4*>(brow) + 1);
+        term(r1, 1u, 4, b47.x);
+        if (keep > 5) term(r1, 2u, 5, b47.y);
+        if (keep > 6) term(r1, 3u, 6, b47.z);
     }
     return __fadd_rn(hi, lo);
 }
@@ -851,9 +854,9 @@ __device__ void sci_decode_controls(const DeviceAsset& a, const LeafEntry& e, ui
     const int keep = (int)((hdr >> 2) & 0x3Fu) + 1;
     const float* brow = a.basis + (uint64_t)t * 64u;
     if (keep <= 7 && base + 4u + (uint64_t)(64 * (keep + 1)) + 4u <= 4ull * a.g.payload_words) {
-        // the coarse block lies inside the payload: word-window reads, terms read once per lane
-        const SciTerms tm(a, t, keep);
-        for (int c = lane; c < 64; c += nl) s_ctrl[c] = sci_control_fast(a.payload, base + 4u + (uint64_t)c * (keep + 1), keep, tm);
+        // the coarse block lies inside the payload
+        const uint32_t* lw = a.payload + e.word_off;
+        for (int c = lane; c < 64; c += nl) s_ctrl[c] = sci_control_fast(lw, 4u + (uint32_t)(c * (keep + 1)), keep, brow, a.scales);
     } else {
         for (int c = lane; c < 64; c += nl) s_ctrl[c] = sci_control(a, rd, base, keep, c, brow);
     }
@@ -1185,408 +1188,9 @@ void launch_decode_cache_plain(const DeviceAsset& a, int frame, float* out, cuda
     decode_plain_kernel<<<a.g.leaf_count, 64, 0, s>>>(a, frame, out);
 }
 
-// ---------------------------------------------------------------------------------------------
-// (c) point queries: one thread per query, decoding only the corner controls it needs.
-
-__device__ __forceinline__ float rt_point(const DeviceAsset& a, const LeafEntry& e, int w, int h, int d, int lx, int ly, int lz,
-                          int frame)
-{
-    const uint32_t* __restrict__ pw = a.payload;
-    const uint64_t base = 4ull * e.word_off;
-    const int total = (int)a.g.frames;
-    const uint32_t cres = (e.header >> 6) & 7u, fres = (e.header >> 9) & 7u;
-    const uint32_t bin8 = time_bin(frame, 8u, total);
-    auto sample = [&](const StreamRef& s, uint32_t res) -> float {
-        if (res == 0u) return 0.0f;
-        if (res == 1u) return decode_control(pw, s, 0, frame, bin8);
-        const AxisWeight ax = g_axis[axis_index(res, w, lx)], ay = g_axis[axis_index(res, h, ly)],
-                         az = g_axis[axis_index(res, d, lz)];
-        const uint32_t r = res;
-        auto at = [&](uint32_t ix, uint32_t iy, uint32_t iz) { return decode_control(pw, s, (iz * r + iy) * r + ix, frame, bin8); };
-        const float c00 = lerp_ref(at(ax.i0, ay.i0, az.i0), at(ax.i1, ay.i0, az.i0), ax.t, ax.omt);
-        const float c01 = lerp_ref(at(ax.i0, ay.i0, az.i1), at(ax.i1, ay.i0, az.i1), ax.t, ax.omt);
-        const float c10 = lerp_ref(at(ax.i0, ay.i1, az.i0), at(ax.i1, ay.i1, az.i0), ax.t, ax.omt);
-        const float c11 = lerp_ref(at(ax.i0, ay.i1, az.i1), at(ax.i1, ay.i1, az.i1), ax.t, ax.omt);
-        return lerp_ref(lerp_ref(c00, c10, ay.t, ay.omt), lerp_ref(c01, c11, ay.t, ay.omt), az.t, az.omt);
-    };
-    StreamRef cs{base + 8u, cres * cres * cres, 8u, e.kf & 0xFFFFu, (e.header >> 2) & 3u};
-    float v = sample(cs, cres);
-    const uint32_t vox = (uint32_t)((lz * 8 + ly) * 8 + lx);
-    bool in_occ = false;
-    uint64_t mask = 0;
-    uint32_t pref = 0;
-    if (e.info & kFlagOccClamp) {
-        const uint64_t ob = base + 8u + e.coarse_bytes;
-        const uint32_t g = vox >> 6;
-        mask = ((uint64_t)ldw(pw, (uint32_t)((ob + 8u * g + 4u) >> 2)) << 32) | ldw(pw, (uint32_t)((ob + 8u * g) >> 2));
-        pref = (ldw(pw, (uint32_t)((ob + 64u + 2u * g) >> 2)) >> ((g & 1u) * 16u)) & 0xFFFFu;
-        in_occ = (mask >> (vox & 63u)) & 1ull;
-    }
-    if (e.info & kFlagFine) {
-        StreamRef fs{base + 8u + e.coarse_bytes, fres * fres * fres, 8u, e.kf >> 16, (e.header >> 4) & 3u};
-        v = __fadd_rn(v, sample(fs, fres));
-    } else if ((e.info & kFlagShell) && in_occ) {
-        StreamRef ss{base + e.shell_off, entry_shell_active(e), 4u, e.kf >> 16, (e.header >> 4) & 3u};
-        const uint32_t di = (pref + __popcll(mask & ((1ull << (vox & 63u)) - 1ull))) & 0xFFFFu;
-        v = __fadd_rn(v, decode_control(pw, ss, di, frame, time_bin(frame, 4u, total)));
-    }
-    if ((e.info & kFlagOccClamp) && !in_occ && v < 0.0f) v = 0.0f;
-    return v;
-}
-
-// The point decode of a scientific leaf whose coarse block and sparse-event section lie inside the
-// payload (so none of the SciReader's per-byte checks can fire) and whose keep is at most 8: the
-// same arithmetic as sci_point's coarse part and sci_sparse, in the same order, with each
-// control's record (at most 8 bytes: keep <= 7) read as two 32-bit windows, the basis row and AC
-// scales read once per query, and the event keys as 32-bit windows.  Returns false (nothing
-// decoded) when the leaf is not of that shape; sci_point then decodes it.
-__device__ __forceinline__ bool sci_point_fast(const DeviceAsset& a, const LeafEntry& e, uint32_t lx, uint32_t ly,
-                                               uint32_t lz, uint32_t t, float& value)
-{
-    const uint32_t hdr = e.header;
-    const int keep = (int)((hdr >> 2) & 0x3Fu) + 1;
-    const uint32_t mode = hdr & 3u;
-    const uint64_t base = 4ull * e.word_off;
-    const uint64_t bytes = 4ull * a.g.payload_words;
-    const uint64_t sb = base + 4u + (uint64_t)(64 * (keep + 1));
-    if (keep > 7 || mode >= 2u || sb + 4u > bytes) return false;
-    const uint32_t* __restrict__ pw = a.payload;
-    const SciTerms tm(a, t, keep);
-    auto at = [&](int ci) { return sci_control_fast(pw, base + 4u + (uint64_t)ci * (keep + 1), keep, tm); };
-    const AxisWeight ax = c_sci_axis[0][lx], ay = c_sci_axis[0][ly], az = c_sci_axis[0][lz];
-    auto ci = [&](int cx, int cy, int cz) { return at((cz * 4 + cy) * 4 + cx); };
-    const float c00 = lerp_ref(ci(ax.i0, ay.i0, az.i0), ci(ax.i1, ay.i0, az.i0), ax.t, ax.omt);
-    const float c01 = lerp_ref(ci(ax.i0, ay.i0, az.i1), ci(ax.i1, ay.i0, az.i1), ax.t, ax.omt);
-    const float c10 = lerp_ref(ci(ax.i0, ay.i1, az.i0), ci(ax.i1, ay.i1, az.i0), ax.t, ax.omt);
-    const float c11 = lerp_ref(ci(ax.i0, ay.i1, az.i1), ci(ax.i1, ay.i1, az.i1), ax.t, ax.omt);
-    const float coarse = lerp_ref(lerp_ref(c00, c10, ay.t, ay.omt), lerp_ref(c01, c11, ay.t, ay.omt), az.t, az.omt);
-    float r = 0.0f;
-    const uint32_t count = (hdr >> 16) & 0x0FFFu;
-    if (mode == 1u && count != 0u) {   // sci_sparse
-        const uint32_t tier = (hdr >> 8) & 3u;
-        const uint32_t cap = tier == 0u ? 64u : tier == 1u ? 256u : tier == 2u ? 768u : 1024u;
-        if (sb + 100u + 2u * cap + cap / 2u + 4u > bytes) return false;   // the section's extent
-        const uint32_t li = (lz * 8u + ly) * 8u + lx;
-        const uint32_t fpb = ((hdr >> 10) & 0xFu) + 1u;
-        const uint32_t bin = t / fpb < 15u ? t / fpb : 15u;
-        const uint32_t lt = (t - bin * fpb) & 0xFFu;
-        const float es = __uint_as_float(pay_u32(pw, sb));
-        const uint32_t mw = pay_u32(pw, sb + 4u + (li >> 5) * 4u);
-        if (es > 0.0f && (mw & (1u << (li & 31u))) != 0u) {
-            const uint64_t bb = sb + 68u;
-            const uint32_t se = pay_u32(pw, bb + bin * 2u);
-            const uint32_t start = se & 0xFFFFu;
-            const uint32_t end = bin + 1u < 16u ? se >> 16 : (count & 0xFFFFu);
-            const uint64_t cb = bb + 32u, rb = cb + cap * 2u;
-            const uint32_t target = ((lt << 9) | (li & 0x1FFu)) & 0xFFFFu;
-            int left = (int)start, right = (int)end - 1;
-            while (left <= right) {
-                const int mid = (left + right) >> 1;
-                const uint32_t key = pay_u32(pw, cb + (uint32_t)mid * 2u) & 0xFFFFu;
-                if (key == target) {
-                    const uint32_t byte = pay_u32(pw, rb + (uint32_t)(mid >> 1)) & 0xFFu;
-                    int q = (int)((mid & 1) == 0 ? (byte & 0xFu) : ((byte >> 4) & 0xFu));
-                    if (q & 8) q -= 16;
-                    r = __fmul_rn((float)q, es);
-                    break;
-                }
-                if (key < target) left = mid + 1;
-                else right = mid - 1;
-            }
-        }
-    }
-    value = __fadd_rn(coarse, r);
-    return true;
-}
-
-__device__ __forceinline__ float sci_point(const DeviceAsset& a, const LeafEntry& e, uint32_t lx, uint32_t ly, uint32_t lz, uint32_t t,
-                           bool& oob)
-{
-    SciReader rd{a.payload, a.g.payload_words, false};
-    const uint64_t base = 4ull * e.word_off;
-    const uint32_t hdr = e.header;
-    const int keep = (int)((hdr >> 2) & 0x3Fu) + 1;
-    const float* brow = a.basis + (uint64_t)t * 64u;
-    const AxisWeight ax = c_sci_axis[0][lx], ay = c_sci_axis[0][ly], az = c_sci_axis[0][lz];
-    auto at = [&](int cx, int cy, int cz) { return sci_control(a, rd, base, keep, (cz * 4 + cy) * 4 + cx, brow); };
-    const float c00 = lerp_ref(at(ax.i0, ay.i0, az.i0), at(ax.i1, ay.i0, az.i0), ax.t, ax.omt);
-    const float c01 = lerp_ref(at(ax.i0, ay.i0, az.i1), at(ax.i1, ay.i0, az.i1), ax.t, ax.omt);
-    const float c10 = lerp_ref(at(ax.i0, ay.i1, az.i0), at(ax.i1, ay.i1, az.i0), ax.t, ax.omt);
-    const float c11 = lerp_ref(at(ax.i0, ay.i1, az.i1), at(ax.i1, ay.i1, az.i1), ax.t, ax.omt);
-    const float coarse = lerp_ref(lerp_ref(c00, c10, ay.t, ay.omt), lerp_ref(c01, c11, ay.t, ay.omt), az.t, az.omt);
-    const uint32_t mode = hdr & 3u;
-    float r = 0.0f;
-    if (mode == 1u) {
-        r = sci_sparse(rd, base, hdr, keep, (lz * 8u + ly) * 8u + lx, t);
-    } else if (mode >= 2u) {
-        const int res = mode == 2u ? 3 : 4;
-        const int bits = (int)((hdr >> 8) & 0xFu);
-        const uint32_t sub = (hdr >> 12) & 7u;
-        const int per = res * res * res;
-        const uint64_t scales = base + 4u + (uint64_t)(64 * (keep + 1));
-        const int gi = mode == 2u ? 1 : 2;
-        const AxisWeight dx = c_sci_axis[gi][lx], dy = c_sci_axis[gi][ly], dz = c_sci_axis[gi][lz];
-        auto tri = [&](uint64_t data, float sc) {
-            auto S = [&](int cx, int cy, int cz) { return bfp_sample(rd, data, res, bits, sc, (cz * res + cy) * res + cx); };
-            const float d00 = lerp_ref(S(dx.i0, dy.i0, dz.i0), S(dx.i1, dy.i0, dz.i0), dx.t, dx.omt);
-            const float d01 = lerp_ref(S(dx.i0, dy.i0, dz.i1), S(dx.i1, dy.i0, dz.i1), dx.t, dx.omt);
-            const float d10 = lerp_ref(S(dx.i0, dy.i1, dz.i0), S(dx.i1, dy.i1, dz.i0), dx.t, dx.omt);
-            const float d11 = lerp_ref(S(dx.i0, dy.i1, dz.i1), S(dx.i1, dy.i1, dz.i1), dx.t, dx.omt);
-            return lerp_ref(lerp_ref(d00, d10, dy.t, dy.omt), lerp_ref(d01, d11, dy.t, dy.omt), dz.t, dz.omt);
-        };
-        if (sub == 1u) {
-            const int tkeep = (int)((hdr >> 15) & 0xFu) + 1;
-            if (bits > 0) {
-                const int bbytes = (per * bits + 7) / 8;
-                const uint64_t data = scales + (uint64_t)(tkeep * 2);
-                for (int k = 0; k < tkeep; ++k) {
-                    const float sc = half_bits_to_float(rd.u16(scales + (uint64_t)(k * 2)));
-                    r = __fadd_rn(r, __fmul_rn(tri(data + (uint64_t)(k * bbytes), sc), __ldg(brow + k)));
-                }
-            }
-        } else {
-            const int fbytes = (per * bits + 7) / 8;
-            const float sc = half_bits_to_float(rd.u16(scales + t * 2u));
-            r = tri(scales + (uint64_t)a.g.frames * 2u + (uint64_t)t * fbytes, sc);
-        }
-    }
-    oob |= rd.oob;
-    return __fadd_rn(coarse, r);
-}
-
-// One point query (x, y, z, t) of one asset; decode errors go to `err`.
-__device__ __forceinline__ float point_value(const DeviceAsset& a, uint4 qq, unsigned long long* err)
-{
-    const uint32_t x = qq.x, y = qq.y, z = qq.z, t = qq.w;
-    // leaf lookup as render/src/vbt_file.cpp:250-262 leafIndexForVoxel (clamped leaf coordinates)
-    const uint32_t bx = min(a.g.lcx - 1u, x >> 3), by = min(a.g.lcy - 1u, y >> 3), bz = min(a.g.lcz - 1u, z >> 3);
-    const uint32_t leaf = (bz * a.g.lcy + by) * a.g.lcx + bx;
-    const LeafEntry e = a.entries[leaf];
-    const uint32_t st = entry_status(e);
-    if (st != kOk) {
-        record_error(err, leaf, st);
-        return 0.0f;
-    }
-    if (a.g.profile == 2u) {
-        if (t >= a.g.frames) {   // the reference indexes its per-frame tables out of range here
-            record_error(err, leaf, kErrDecodeOob);
-            return 0.0f;
-        }
-        float fv;
-        if (sci_point_fast(a, e, x & 7u, y & 7u, z & 7u, t, fv)) return fv;
-        bool oob = false;
-        const float v = sci_point(a, e, x & 7u, y & 7u, z & 7u, t, oob);
-        if (oob) record_error(err, leaf, kErrDecodeOob);
-        return v;
-    }
-    if ((e.header & 3u) == kModeEmpty) return 0.0f;
-    uint32_t gx, gy, gz;
-    int w, h, d;
-    leaf_extent(a.g, leaf, gx, gy, gz, w, h, d);
-    const int lx = (int)(x - bx * 8u), ly = (int)(y - by * 8u), lz = (int)(z - bz * 8u);
-    if (lx >= w || ly >= h || lz >= d) return 0.0f;   // outside the volume: no such voxel in any frame
-    return rt_point(a, e, w, h, d, lx, ly, lz, clamp_frame((int)t, (int)a.g.frames));
-}
-
-// True when point_value returns 0 without decoding anything and without recording an error: a
-// render-temporal query in an EMPTY leaf or outside the volume.
-__device__ __forceinline__ bool point_trivial(const DeviceAsset& a, uint4 qq)
-{
-    if (a.g.profile == 2u) return false;
-    const uint32_t bx = min(a.g.lcx - 1u, qq.x >> 3), by = min(a.g.lcy - 1u, qq.y >> 3), bz = min(a.g.lcz - 1u, qq.z >> 3);
-    const uint32_t leaf = (bz * a.g.lcy + by) * a.g.lcx + bx;
-    const uint32_t info = __ldg(&a.entries[leaf].info), header = __ldg(&a.entries[leaf].header);
-    if (((info >> 16) & 0xFFu) != kOk) return false;   // point_value records the status
-    if ((header & 3u) == kModeEmpty) return true;
-    uint32_t gx, gy, gz;
-    int w, h, d;
-    leaf_extent(a.g, leaf, gx, gy, gz, w, h, d);
-    return (int)(qq.x - bx * 8u) >= w || (int)(qq.y - by * 8u) >= h || (int)(qq.z - bz * 8u) >= d;
-}
-
-// Point queries in chunks of `per` x 128 per CTA.  In a chunk of a sparse volume a first pass
-// answers the trivial queries (EMPTY leaf, outside the volume) and passes the others to a
-// shared-memory list that the CTA's warps then decode with every lane busy -- most random queries
-// there are trivial, and a warp that decoded its few non-trivial lanes in place would leave the
-// rest idle.  Chunks of other volumes decode every query in place.  Values are point_value's
-// either way.  `per` is chosen on the host so that the grid still fills the GPU.
-constexpr int kPqThreads = 128, kPqMaxPer = 8, kPqMaxChunk = kPqThreads * kPqMaxPer;
-
-template <class Resolve>
-__device__ __forceinline__ void query_chunk(uint64_t n, int per, const uint4* __restrict__ q, const Resolve& resolve)
-{
-    __shared__ uint32_t s_list[kPqMaxChunk];
-    __shared__ uint32_t s_count;
-    const int tid = threadIdx.x, lane = tid & 31;
-    const uint64_t base = (uint64_t)blockIdx.x * (uint64_t)(per * kPqThreads);
-    if (!resolve.sparse(base)) {   // a chunk of a mostly active volume: each thread its own queries
-        for (int r = 0; r < per; ++r) {
-            const uint64_t i = base + (uint64_t)(r * kPqThreads + tid);
-            if (i < n) resolve.second(i, q[i]);
-        }
-        return;
-    }
-    if (tid == 0) s_count = 0u;
-    __syncthreads();
-    for (int r = 0; r < per; ++r) {
-        const uint32_t j = (uint32_t)(r * kPqThreads + tid);
-        const uint64_t i = base + j;
-        bool need = false;
-        uint4 qq = make_uint4(0u, 0u, 0u, 0u);
-        if (i < n) {
-            qq = q[i];
-            need = resolve.first(i, qq);
-        }
-        const unsigned m = __ballot_sync(0xFFFFFFFFu, need);
-        uint32_t wbase = 0u;
-        if (lane == 0 && m) wbase = atomicAdd(&s_count, (uint32_t)__popc(m));
-        wbase = __shfl_sync(0xFFFFFFFFu, wbase, 0);
-        if (need) s_list[wbase + (uint32_t)__popc(m & ((1u << lane) - 1u))] = j;
-    }
-    __syncthreads();
-    const uint32_t cnt = s_count;
-    for (uint32_t k = (uint32_t)tid; k < cnt; k += kPqThreads) {
-        const uint64_t i = base + s_list[k];
-        resolve.second(i, q[i]);
-    }
-}
-
-// Queries per thread: the largest of 8, 4, 2, 1 that still gives four CTAs per SM.
-static int query_per_thread(uint64_t n)
-{
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const uint64_t want = 4ull * (uint64_t)(sms > 0 ? sms : 1);
-    int per = kPqMaxPer;
-    while (per > 1 && (n + (uint64_t)per * kPqThreads - 1) / ((uint64_t)per * kPqThreads) < want) per >>= 1;
-    return per;
-}
-
-struct OneAssetQueries {
-    const DeviceAsset& a;
-    float* __restrict__ out;
-    __device__ __forceinline__ bool sparse(uint64_t) const { return a.g.sparse != 0u; }
-    __device__ __forceinline__ bool first(uint64_t i, uint4 qq) const
-    {
-        if (!point_trivial(a, qq)) return true;
-        out[i] = 0.0f;
-        return false;
-    }
-    __device__ __forceinline__ void second(uint64_t i, uint4 qq) const { out[i] = point_value(a, qq, a.err); }
-};
-
-// One thread per query: the shape for volumes whose leaves are mostly active.
-__global__ void __launch_bounds__(128) query_points_kernel(DeviceAsset a, const uint32_t* __restrict__ q, uint64_t n,
-                                                           float* __restrict__ out)
-{
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    out[i] = point_value(a, reinterpret_cast<const uint4*>(q)[i], a.err);
-}
-
-// Compacted chunks: the shape for sparse volumes.
-__global__ void __launch_bounds__(kPqThreads) query_points_compact_kernel(const __grid_constant__ DeviceAsset a,
-                                                                          const uint32_t* __restrict__ q, uint64_t n,
-                                                                          int per, float* __restrict__ out)
-{
-    query_chunk(n, per, reinterpret_cast<const uint4*>(q), OneAssetQueries{a, out});
-}
-
-// Point queries of several requests over several resident assets in one launch.  The segment
-// table holds starts[0..k] (each request's first query; starts[k] = n), asset[k] (request r reads
-// assets[asset[r]]) and, 8-byte aligned after them, outs[k] (request r's result array).  Request
-// r's decode errors go to errs[r].
-struct BatchQueries {
-    const DeviceAsset* __restrict__ assets;
-    const uint32_t* __restrict__ seg;
-    uint32_t k;
-    unsigned long long* errs;
-    __device__ __forceinline__ int request(uint64_t i) const
-    {
-        int lo = 0, hi = (int)k - 1;
-        while (lo < hi) {   // the last request whose first query is at or before i
-            const int mid = (lo + hi + 1) >> 1;
-            if (__ldg(seg + mid) <= (uint32_t)i) lo = mid;
-            else hi = mid - 1;
-        }
-        return lo;
-    }
-    // the chunk starting at query i takes the compacting path when its first query's asset is sparse
-    __device__ __forceinline__ bool sparse(uint64_t i) const
-    {
-        return assets[__ldg(seg + k + 1 + request(i))].g.sparse != 0u;
-    }
-    __device__ __forceinline__ void put(int r, uint64_t i, float v) const
-    {
-        const unsigned long long* outs = reinterpret_cast<const unsigned long long*>(seg + ((2u * k + 2u) & ~1u));
-        reinterpret_cast<float*>(__ldg(outs + r))[i - __ldg(seg + r)] = v;
-    }
-    __device__ __forceinline__ bool first(uint64_t i, uint4 qq) const
-    {
-        const int r = request(i);
-        if (!point_trivial(assets[__ldg(seg + k + 1 + r)], qq)) return true;
-        put(r, i, 0.0f);
-        return false;
-    }
-    __device__ __forceinline__ void second(uint64_t i, uint4 qq) const
-    {
-        const int r = request(i);
-        put(r, i, point_value(assets[__ldg(seg + k + 1 + r)], qq, errs + r));
-    }
-};
-
-__global__ void __launch_bounds__(128) query_points_batch_kernel(const DeviceAsset* __restrict__ assets,
-                                                                 const uint32_t* __restrict__ seg, uint32_t k,
-                                                                 const uint4* __restrict__ q, uint64_t n,
-                                                                 unsigned long long* errs)
-{
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int lo = 0, hi = (int)k - 1;
-    while (lo < hi) {   // the last request whose first query is at or before i
-        const int mid = (lo + hi + 1) >> 1;
-        if (__ldg(seg + mid) <= (uint32_t)i) lo = mid;
-        else hi = mid - 1;
-    }
-    const unsigned long long* outs = reinterpret_cast<const unsigned long long*>(seg + ((2u * k + 2u) & ~1u));
-    float* o = reinterpret_cast<float*>(__ldg(outs + lo));
-    o[i - __ldg(seg + lo)] = point_value(assets[__ldg(seg + k + 1 + lo)], q[i], errs + lo);
-}
-
-__global__ void __launch_bounds__(kPqThreads) query_points_batch_compact_kernel(
-    const DeviceAsset* __restrict__ assets, const uint32_t* __restrict__ seg, uint32_t k, const uint4* __restrict__ q,
-    uint64_t n, int per, unsigned long long* errs)
-{
-    query_chunk(n, per, q, BatchQueries{assets, seg, k, errs});
-}
-
-void launch_query_points_batch(const DeviceAsset* assets, const uint32_t* seg, uint32_t k, const uint4* q, uint64_t n,
-                               unsigned long long* errs, int sparse, cudaStream_t s)
-{
-    if (n == 0 || k == 0) return;
-    if (sparse == 0) {
-        query_points_batch_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(assets, seg, k, q, n, errs);
-        return;
-    }
-    // with requests on mostly active volumes in the launch, one query per thread for their chunks
-    const int per = sparse == 2 ? query_per_thread(n) : 1;
-    const uint64_t chunk = (uint64_t)per * kPqThreads;
-    query_points_batch_compact_kernel<<<(unsigned)((n + chunk - 1) / chunk), kPqThreads, 0, s>>>(assets, seg, k, q, n,
-                                                                                                   per, errs);
-}
-
-void launch_query_points(const DeviceAsset& a, const uint32_t* q, uint64_t n, float* out, bool sparse, cudaStream_t s)
-{
-    if (n == 0) return;
-    if (!sparse) {
-        query_points_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(a, q, n, out);
-        return;
-    }
-    const int per = query_per_thread(n);
-    const uint64_t chunk = (uint64_t)per * kPqThreads;
-    query_points_compact_kernel<<<(unsigned)((n + chunk - 1) / chunk), kPqThreads, 0, s>>>(a, q, n, per, out);
-}
+}  // namespace vbtb
+#include "point_query.cuh"
+namespace vbtb {
 
 // Z-slice over [t0, t1): one warp per (leaf of the z layer, frame); lanes 0..7 produce rows.
 __global__ void __launch_bounds__(kDecodeWarps * 32) query_slice_kernel(DeviceAsset a, uint32_t z, int t0, int t1,

@@ -14,6 +14,8 @@
 // (kernel a), so no read here can leave the leaf: keyframe indices stay in [keyStart,
 // keyStart + keyCount) and keyStart + keyCount <= keyframe count was checked for every control.
 #pragma once
+#include <cuda_fp16.h>
+
 #include "vbt_format.cuh"
 
 namespace vbtb {
@@ -86,7 +88,9 @@ __device__ __forceinline__ void key_read(const uint32_t* __restrict__ pw, uint64
 __device__ __forceinline__ uint32_t time_bin(int frame, uint32_t bins, int total)
 {
     if (bins == 0u) return 0u;
-    const uint32_t q = (uint32_t)(((long long)frame * bins) / (total > 1 ? total : 1));
+    const uint32_t n = (uint32_t)(total > 1 ? total : 1);
+    // 0 <= frame < total: the product fits 32 bits for any real frame count (bins <= 8)
+    const uint32_t q = n < (1u << 28) ? (uint32_t)frame * bins / n : (uint32_t)(((long long)frame * bins) / n);
     return q < bins - 1u ? q : bins - 1u;
 }
 
@@ -157,6 +161,86 @@ __device__ __forceinline__ float decode_control(const uint32_t* __restrict__ pw,
     if (moved_lo) v0 = key_value(pw, kb, s.codec, ks + lo);
     const float alpha = __fdiv_rn((float)(frame - f0), (float)(f1 - f0));
     return __fadd_rn(v0, __fmul_rn(alpha, __fsub_rn(v1, v0)));
+}
+
+// binary16 -> binary32 with the hardware conversion; NaNs keep their payload bits exactly as
+// src/render_temporal_decode.cpp:167-199 maps them.
+__device__ __forceinline__ float half_to_float_exact(uint32_t h)
+{
+    const float f = __half2float(__ushort_as_half((unsigned short)h));
+    const bool nan = (h & 0x7C00u) == 0x7C00u && (h & 0x3FFu) != 0u;
+    return nan ? __uint_as_float(((h & 0x8000u) << 16) | 0x7F800000u | ((h & 0x3FFu) << 13)) : f;
+}
+
+// A control stream by its byte offset inside a leaf (32-bit offsets from the leaf's first word).
+struct LeafStream {
+    const uint32_t* __restrict__ w;   // the leaf block
+    uint32_t base, controls, bins, kf;
+};
+
+// Control c of an FP16 stream whose key frames strictly increase, at clamped frame `frame`: the value
+// decode_control's search gives (for such keys the canonical one: the first key's value before it,
+// the last key's after it, the key's on an exact hit, else the lerp of the pair around the frame;
+// see the head of rt_staged.cuh).  Four keys (12 bytes from the hinted one on) are taken at a time
+// as independent word reads and the pair is selected in registers: a time bin rarely spans more, so
+// a control is two dependent steps (descriptor and hint, keys) where the search's halving makes
+// four to seven.  The payload's 16-byte tail padding covers the words past the last key.
+__device__ __forceinline__ float control_sorted(const LeafStream& s, uint32_t c, int frame, uint32_t bin)
+{
+    const uint32_t desc = __ldg(s.w + (s.base >> 2) + c);
+    const uint32_t w0 = __ldg(s.w + ((s.base + 4u * s.controls + c * s.bins + bin) >> 2));
+    const uint32_t kc = (desc >> 16) & 0xFFu, ks = desc & 0xFFFFu;
+    if (kc == 0u || ks + kc > s.kf) return 0.0f;   // see decode_control
+    const uint32_t kb = s.base + s.controls * 4u + align4(s.controls * s.bins) + 3u * ks;
+    const uint32_t hb = (w0 >> ((bin & 3u) * 8u)) & 0xFFu;
+    uint32_t lo = hb < kc - 1u ? hb : kc - 1u;
+    for (;;) {
+        const uint32_t b = kb + 3u * lo;
+        const uint32_t* w = s.w + (b >> 2);
+        const uint32_t sh = (b & 3u) * 8u;
+        const uint32_t x0 = __ldg(w), x1 = __ldg(w + 1), x2 = __ldg(w + 2), x3 = __ldg(w + 3);
+        const uint32_t a0 = __funnelshift_r(x0, x1, sh), a1 = __funnelshift_r(x1, x2, sh),
+                       a2 = __funnelshift_r(x2, x3, sh);
+        const uint32_t left = kc - lo;   // keys from lo on
+        const int f0 = (int)(a0 & 0xFFu), f1 = (int)(a0 >> 24), f2 = (int)((a1 >> 16) & 0xFFu),
+                  f3 = (int)((a2 >> 8) & 0xFFu);
+        const uint32_t h0 = (a0 >> 8) & 0xFFFFu, h1 = a1 & 0xFFFFu, h2 = __byte_perm(a1, a2, 0x0043) & 0xFFFFu,
+                       h3 = a2 >> 16;
+        if (f0 > frame) {
+            if (lo == 0u) return half_to_float_exact(h0);
+            lo = 0u;   // the hint overshot
+            continue;
+        }
+        const bool p1 = left > 1u && f1 <= frame, p2 = left > 2u && p1 && f2 <= frame,
+                   p3 = left > 3u && p2 && f3 <= frame;
+        if (p3 && left > 4u) {   // the pair may lie further on
+            lo += 3u;
+            continue;
+        }
+        const int fp = p3 ? f3 : p2 ? f2 : p1 ? f1 : f0;
+        const float vp = half_to_float_exact(p3 ? h3 : p2 ? h2 : p1 ? h1 : h0);
+        const uint32_t at = p3 ? 3u : p2 ? 2u : p1 ? 1u : 0u;
+        if (fp == frame || at + 1u == left) return vp;   // an exact hit, or past the last key
+        const int fn = p2 ? f3 : p1 ? f2 : f1;
+        const float vn = half_to_float_exact(p2 ? h3 : p1 ? h2 : h1);
+        const float alpha = __fdiv_rn((float)(frame - fp), (float)(fn - fp));
+        return __fadd_rn(vp, __fmul_rn(alpha, __fsub_rn(vn, vp)));
+    }
+}
+
+// The reference's search as a call of its own (leaves with unordered keys or FP32 keys).
+__device__ __noinline__ static float control_searched(const uint32_t* w, uint32_t base, uint32_t controls, uint32_t bins,
+                                                      uint32_t kf, uint32_t codec, uint32_t c, int frame, uint32_t bin)
+{
+    return decode_control(w, StreamRef{base, controls, bins, kf, codec}, c, frame, bin);
+}
+
+// Control c at clamped frame `frame`; sorted: the leaf's kFlagSorted.
+__device__ __forceinline__ float control_at(const LeafStream& s, uint32_t codec, uint32_t c, int frame, uint32_t bin,
+                                            bool sorted)
+{
+    if (sorted && codec != 1u) return control_sorted(s, c, frame, bin);
+    return control_searched(s.w, s.base, s.controls, s.bins, s.kf, codec, c, frame, bin);
 }
 
 // a*(1-t) + b*t with the reference's rounding (two products, one sum; 1-t precomputed exactly).

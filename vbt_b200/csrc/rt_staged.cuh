@@ -43,15 +43,6 @@ __device__ __forceinline__ float2 lerp2(float2 a, float2 b, float2 t, float2 omt
                        __fadd_rn(__fmul_rn(a.y, omt.y), __fmul_rn(b.y, t.y)));
 }
 
-// binary16 -> binary32 with the hardware conversion; NaNs keep their payload bits exactly as
-// src/render_temporal_decode.cpp:167-199 maps them.
-__device__ __forceinline__ float half_to_float_exact(uint32_t h)
-{
-    const float f = __half2float(__ushort_as_half((unsigned short)h));
-    const bool nan = (h & 0x7C00u) == 0x7C00u && (h & 0x3FFu) != 0u;
-    return nan ? __uint_as_float(((h & 0x8000u) << 16) | 0x7F800000u | ((h & 0x3FFu) << 13)) : f;
-}
-
 __device__ __forceinline__ uint32_t row_byte(uint32_t r0, uint32_t r1, uint32_t b)
 {
     return ((b < 4u ? r0 : r1) >> ((b & 3u) * 8u)) & 0xFFu;
