@@ -10,8 +10,8 @@
 //
 // Render-temporal arithmetic is bit-exact with the reference CPU decoder (every float op is an
 // explicitly rounded _rn intrinsic; see rt_search.cuh).  Scientific coarse controls are summed in
-// compensated float-float arithmetic (error-free products and two-sums) to track the reference's
-// double accumulation (render/src/scientific_decode.cpp:82-97) without FP64 on the device.
+// double, as the reference sums them (render/src/scientific_decode.cpp:82-97): a control is a handful
+// of fused multiply-adds, fewer than half the instructions of a compensated float sum.
 #include <cuda/atomic>
 
 #include <mutex>
@@ -26,6 +26,7 @@ __constant__ AxisWeight c_axis[kAxisRes * kAxisExt * kAxisPos];
 __device__ AxisWeight g_axis[kAxisRes * kAxisExt * kAxisPos];
 // Scientific trilinear axes: [0] coarse 4^3 grid (f = x/7*3, clamp 0..2), [1] dense 3^3, [2] dense 4^3.
 __constant__ AxisWeight c_sci_axis[3][8];
+__device__ AxisWeight g_sci_axis[3][8];   // the same, for reads whose index differs from lane to lane
 }  // namespace vbtb
 
 #include <cuda_fp16.h>
@@ -80,6 +81,7 @@ void upload_axis_tables()
             sci[g][p] = AxisWeight{(uint8_t)i0, (uint8_t)(i0 + 1), 0, 0, t, 1.0f - t};
         }
     cudaMemcpyToSymbol(c_sci_axis, sci, sizeof(sci));
+    cudaMemcpyToSymbol(g_sci_axis, sci, sizeof(sci));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -556,22 +558,6 @@ struct SciReader {
     }
 };
 
-// Error-free transforms for the compensated sum.
-__device__ __forceinline__ void two_prod(float a, float b, float& p, float& e)
-{
-    p = __fmul_rn(a, b);
-    e = __fmaf_rn(a, b, -p);
-}
-__device__ __forceinline__ void ff_add(float& hi, float& lo, float ph, float pl)
-{
-    const float s = __fadd_rn(hi, ph);
-    const float bb = __fsub_rn(s, hi);
-    const float err = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bb)), __fsub_rn(ph, bb));
-    const float t = __fadd_rn(__fadd_rn(err, lo), pl);
-    hi = __fadd_rn(s, t);
-    lo = __fsub_rn(t, __fsub_rn(hi, s));
-}
-
 // 32 bits of the payload from byte b, b unaligned (two word reads; the payload's 16-byte tail
 // padding keeps the second word inside the allocation).
 __device__ __forceinline__ uint32_t pay_u32(const uint32_t* __restrict__ pw, uint64_t b)
@@ -588,8 +574,8 @@ __device__ __forceinline__ float byte_to_float(uint32_t word, uint32_t byte)
 }
 
 // sci_control for a record of at most 8 bytes (keep <= 7: DC half in bytes 0-1, AC byte k at byte
-// k + 1) at byte cb of the payload window `w`, inside the payload: the same products and compensated
-// sum in the same order, the record read as words and only the kept terms visited.
+// k + 1) at byte cb of the payload window `w`, inside the payload: the same sum in the same order,
+// the record read as words and only the kept terms visited.
 __device__ __forceinline__ float sci_control_fast(const uint32_t* __restrict__ w, uint32_t cb, int keep,
                                                   const float* __restrict__ brow, const float* __restrict__ scales)
 {
@@ -599,12 +585,9 @@ __device__ __forceinline__ float sci_control_fast(const uint32_t* __restrict__ w
     const uint32_t r0 = __funnelshift_r(__ldg(p), x1, sh);
     const uint32_t r1 = keep > 2 ? __funnelshift_r(x1, __ldg(p + 2), sh) : 0u;
     const float4 b03 = __ldg(reinterpret_cast<const float4*>(brow));   // rows of 64 floats
-    float hi, lo;
-    two_prod(half_to_float_exact(r0 & 0xFFFFu), b03.x, hi, lo);
+    double sum = (double)half_to_float_exact(r0 & 0xFFFFu) * (double)b03.x;
     auto term = [&](uint32_t word, uint32_t byte, int k, float b) {
-        float ph, pl;
-        two_prod(__fmul_rn(byte_to_float(word, byte), __ldg(scales + k - 1)), b, ph, pl);
-        ff_add(hi, lo, ph, pl);
+        sum = __fma_rn((double)__fmul_rn(byte_to_float(word, byte), __ldg(scales + k - 1)), (double)b, sum);
     };
     if (keep > 1) term(r0, 2u, 1, b03.y);
     if (keep > 2) term(r0, 3u, 2, b03.z);
@@ -615,23 +598,22 @@ __device__ __forceinline__ float sci_control_fast(const uint32_t* __restrict__ w
         if (keep > 5) term(r1, 2u, 5, b47.y);
         if (keep > 6) term(r1, 3u, 6, b47.z);
     }
-    return __fadd_rn(hi, lo);
+    return (float)sum;
 }
 
-// Coarse control ci at frame t: DC * b0(t) + sum_k (i8 * acScale[k-1]) * bk(t).
+// Coarse control ci at frame t: DC * b0(t) + sum_k (i8 * acScale[k-1]) * bk(t), summed in double as the
+// reference sums (render/src/scientific_decode.cpp:82-97): a product of two floats is exact in double,
+// so the fused multiply-add rounds as the reference's separate product and sum do.
 __device__ __forceinline__ float sci_control(const DeviceAsset& a, SciReader& rd, uint64_t base, int keep, int ci,
                                              const float* __restrict__ brow)
 {
     const uint64_t cb = base + 4u + (uint64_t)ci * (keep + 1);
-    float hi, lo;
-    two_prod(half_bits_to_float(rd.u16(cb)), __ldg(brow), hi, lo);
+    double sum = (double)half_bits_to_float(rd.u16(cb)) * (double)__ldg(brow);
     for (int k = 1; k < keep; ++k) {
         const float coeff = __fmul_rn((float)(int8_t)rd.byte(cb + 2u + (k - 1)), __ldg(a.scales + k - 1));
-        float ph, pl;
-        two_prod(coeff, __ldg(brow + k), ph, pl);
-        ff_add(hi, lo, ph, pl);
+        sum = __fma_rn((double)coeff, (double)__ldg(brow + k), sum);
     }
-    return __fadd_rn(hi, lo);
+    return (float)sum;
 }
 
 __device__ __forceinline__ float decode_bfp(uint32_t q, float scale, int bits)
@@ -954,84 +936,47 @@ struct FrameList {
     int f[kMaxLaunchFrames];
 };
 
-template <bool DENSE, bool SCI>
+// Leaf per warp (render-temporal caches): the shape the autotuner weighs against the leaf-per-CTA kernel.
 __global__ void __launch_bounds__(kDecodeWarps * 32, 2) decode_kernel(DeviceAsset a, FrameList fl, float* __restrict__ out,
                                                                      uint64_t frame_stride)
 {
     __shared__ __align__(16) float s_ctrl_all[kDecodeWarps][kWarpSlots];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float* s_ctrl = s_ctrl_all[warp];
-    const uint32_t n_items = DENSE ? a.g.leaf_count : *(volatile const uint32_t*)a.counters;
+    const uint32_t n_items = *(volatile const uint32_t*)a.counters;
     const uint32_t warps_total = gridDim.x * kDecodeWarps;
     for (uint32_t item = blockIdx.x * kDecodeWarps + warp; item < n_items; item += warps_total) {
-        const uint32_t leaf = DENSE ? item : __ldg(a.active_list + item);
+        const uint32_t leaf = __ldg(a.active_list + item);
         const LeafEntry e = a.entries[leaf];
         uint32_t bx, by, bz;
         int w, h, d;
         leaf_extent(a.g, leaf, bx, by, bz, w, h, d);
-        const bool empty = !SCI && (e.header & 3u) == kModeEmpty;
+        const bool empty = (e.header & 3u) == kModeEmpty;
         const uint32_t st = entry_status(e);
         if (st != kOk && lane == 0) record_error(a.err, leaf, st);
-        // scientific SparseEvents leaves with sorted keys: events are added by visiting the
-        // frame's bin after the rows are written, instead of one search per voxel
-        const bool scatter = SCI && st == kOk && (e.header & 3u) == 1u && (e.info & kFlagSorted) != 0u;
         for (int fi = 0; fi < fl.n; ++fi) {
-            const int frame = clamp_frame(fl.f[fi], (int)a.g.frames);
-            bool oob = false;
-            if (!empty && st == kOk) {
-                if (SCI) sci_decode_controls(a, e, (uint32_t)fl.f[fi], s_ctrl, lane, oob);
-                else rt_decode_controls(a, e, frame, s_ctrl, lane);
-            }
+            if (!empty && st == kOk) rt_decode_controls(a, e, clamp_frame(fl.f[fi], (int)a.g.frames), s_ctrl, lane);
             __syncwarp();
             for (int r = lane; r < 64; r += 32) {
-                const int ly = r & 7, lz = r >> 3;
                 float v[8];
                 if (empty || st != kOk) {
 #pragma unroll
                     for (int i = 0; i < 8; ++i) v[i] = 0.0f;
-                } else if (SCI) {
-                    sci_row(a, e, s_ctrl, (uint32_t)fl.f[fi], w, h, d, ly, lz, v, oob, scatter);
                 } else {
-                    rt_row(a, e, s_ctrl, w, h, d, ly, lz, v);
+                    rt_row(a, e, s_ctrl, w, h, d, r & 7, r >> 3, v);
                 }
-                if (DENSE) {
-                    if (ly < h && lz < d) {
-                        float* dst = out + (uint64_t)fi * frame_stride +
-                                     ((uint64_t)(bz * 8 + lz) * a.g.height + (by * 8 + ly)) * a.g.width + bx * 8;
-                        if (w == 8 && (((uintptr_t)dst) & 15u) == 0u) {
-                            reinterpret_cast<float4*>(dst)[0] = make_float4(v[0], v[1], v[2], v[3]);
-                            reinterpret_cast<float4*>(dst)[1] = make_float4(v[4], v[5], v[6], v[7]);
-                        } else {
-                            for (int i = 0; i < w; ++i) dst[i] = v[i];
-                        }
-                    }
-                } else {
-                    float4* dst = reinterpret_cast<float4*>(out + (uint64_t)fi * frame_stride + (uint64_t)item * 512u + r * 8);
-                    dst[0] = make_float4(v[0], v[1], v[2], v[3]);
-                    dst[1] = make_float4(v[4], v[5], v[6], v[7]);
-                }
+                float4* dst = reinterpret_cast<float4*>(out + (uint64_t)fi * frame_stride + (uint64_t)item * 512u + r * 8);
+                dst[0] = make_float4(v[0], v[1], v[2], v[3]);
+                dst[1] = make_float4(v[4], v[5], v[6], v[7]);
             }
-            if (scatter && (uint32_t)fl.f[fi] < a.g.frames) {
-                __syncwarp();   // the rows written by the other lanes are visible
-                if (DENSE) {
-                    float* fb = out + (uint64_t)fi * frame_stride;
-                    sci_scatter_frame(a, e, (uint32_t)fl.f[fi], w, h, d, lane,
-                                      [&](uint32_t li) {
-                                          return fb + ((uint64_t)(bz * 8 + (li >> 6)) * a.g.height +
-                                                       (by * 8 + ((li >> 3) & 7u))) * a.g.width + bx * 8 + (li & 7u);
-                                      },
-                                      oob);
-                } else {
-                    float* fb = out + (uint64_t)fi * frame_stride + (uint64_t)item * 512u;
-                    sci_scatter_frame(a, e, (uint32_t)fl.f[fi], w, h, d, lane, [&](uint32_t li) { return fb + li; },
-                                      oob);
-                }
-            }
-            if (__any_sync(0xFFFFFFFFu, oob) && lane == 0) record_error(a.err, leaf, kErrDecodeOob);
             __syncwarp();
         }
     }
 }
+
+}  // namespace vbtb
+#include "sci_frames.cuh"
+namespace vbtb {
 
 // Render-temporal decode kernel (TMA-staged leaf, one CTA per leaf): rt_kernel_leaf.cuh
 }  // namespace vbtb
@@ -1045,7 +990,7 @@ static int default_grid()
         int dev = 0, sms = 0, per = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, decode_kernel<false, false>, kDecodeWarps * 32, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, decode_kernel, kDecodeWarps * 32, 0);
         g = sms * (per > 0 ? per : 1);
     }
     return g;
@@ -1058,7 +1003,7 @@ void launch_decode_cache(const DeviceAsset& a, uint32_t seq, const int* frames, 
     fl.n = nframes;
     for (int i = 0; i < nframes; ++i) fl.f[i] = frames[i];
     if (a.g.profile == 2u)
-        decode_kernel<false, true><<<grid > 0 ? grid : default_grid(), kDecodeWarps * 32, 0, s>>>(a, fl, out, stride);
+        launch_sci_frames<false>(a, fl, out, stride, grid, s);
     else
         launch_rt_leaf(a, seq, fl, out, stride, grid, false, s);
 }
@@ -1126,7 +1071,7 @@ void launch_decode_dense(const DeviceAsset& a, uint32_t seq, const int* frames, 
     for (int i = 0; i < nframes; ++i) fl.f[i] = frames[i];
     const uint64_t stride = (uint64_t)a.g.width * a.g.height * a.g.depth;
     if (a.g.profile == 2u)
-        decode_kernel<true, true><<<grid > 0 ? grid : default_grid(), kDecodeWarps * 32, 0, s>>>(a, fl, out, stride);
+        launch_sci_frames<true>(a, fl, out, stride, grid, s);
     else
         launch_rt_leaf(a, seq, fl, out, stride, grid, true, s);
 }
@@ -1139,9 +1084,8 @@ void launch_decode_cache_warp(const DeviceAsset& a, const int* frames, int nfram
     FrameList fl{};
     fl.n = nframes;
     for (int i = 0; i < nframes; ++i) fl.f[i] = frames[i];
-    const int g = grid > 0 ? grid : default_grid();
-    if (a.g.profile == 2u) decode_kernel<false, true><<<g, kDecodeWarps * 32, 0, s>>>(a, fl, out, stride);
-    else decode_kernel<false, false><<<g, kDecodeWarps * 32, 0, s>>>(a, fl, out, stride);
+    if (a.g.profile == 2u) launch_sci_frames<false>(a, fl, out, stride, grid, s);
+    else decode_kernel<<<grid > 0 ? grid : default_grid(), kDecodeWarps * 32, 0, s>>>(a, fl, out, stride);
 }
 
 int decode_warp_grid() { return default_grid(); }

@@ -381,7 +381,7 @@ __device__ __forceinline__ void query_chunk(uint64_t n, uint32_t chunk, const ui
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     if (threadIdx.x < 32u) {
         const int g = (int)(lane >> 3), p = (int)(lane & 7u);
-        const AxisWeight w = g < 2 ? g_axis[axis_index(g == 0 ? 4 : 6, 8, p)] : c_sci_axis[g - 2][p];
+        const AxisWeight w = g < 2 ? g_axis[axis_index(g == 0 ? 4 : 6, 8, p)] : g_sci_axis[g - 2][p];
         s_axis[lane] = make_float2(w.t, __uint_as_float((uint32_t)w.i0));
     }
     __syncthreads();
