@@ -476,7 +476,7 @@ int vbt_decode_cache(vbt_asset* a, const int* frames, int nframes, float* out, u
     if (st) return st;
     DeviceGuard guard(a->device);
     launch_decode_cache(a->dev, a->launch_seq.fetch_add(1), frames, nframes, out, stride, grid, static_cast<cudaStream_t>(stream));
-    return check_launch("decode_kernel<cache>");
+    return check_launch("cache decode");
 }
 
 int vbt_decode_control_cache(vbt_asset* a, const int* frames, int nframes, float* out, uint64_t stride, void* stream)
@@ -508,7 +508,7 @@ int vbt_decode_frames(vbt_asset* a, const int* frames, int nframes, float* out, 
     if (st) return st;
     DeviceGuard guard(a->device);
     launch_decode_dense(a->dev, a->launch_seq.fetch_add(1), frames, nframes, out, grid, static_cast<cudaStream_t>(stream));
-    return check_launch("decode_kernel<dense>");
+    return check_launch("dense decode");
 }
 
 int vbt_query_points(vbt_asset* a, const uint32_t* q, uint64_t n, float* out, void* stream)
@@ -577,7 +577,7 @@ int vbt_decode_frames_host(vbt_asset* a, const int* frames, int nframes, float* 
     if ((st = grow(&a->stage_out, &a->stage_out_bytes, 4ull * vox * nframes))) return st;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     launch_decode_dense(a->dev, a->launch_seq.fetch_add(1), frames, nframes, static_cast<float*>(a->stage_out), 0, s);
-    if ((st = check_launch("decode_kernel<dense>"))) return st;
+    if ((st = check_launch("dense decode"))) return st;
     CUDA_TRY(cudaMemcpyAsync(out, a->stage_out, 4ull * vox * nframes, cudaMemcpyDeviceToHost, s));
     return vbt_asset_sync_status(a, stream, nullptr);
 }
@@ -592,7 +592,7 @@ int vbt_decode_window(vbt_asset* a, int t0, int n, float* d_out, uint64_t frame_
             return fail(VBT_STATUS_INVALID_ARGUMENT, "frame_stride below leaf_count * 512");
         DeviceGuard guard(a->device);
         launch_sci_window(a->dev, t0, n, d_out, frame_stride, static_cast<cudaStream_t>(stream));
-        return check_launch("sci_window_kernel");
+        return check_launch("sci_frames_kernel");
     }
     if (n < 1 || n > 64 || t0 < 0 || (uint64_t)t0 + (uint64_t)n > a->hdr.frames)
         return fail(VBT_STATUS_INVALID_ARGUMENT, "render windows must cover 1..64 frames inside [0, frames)");

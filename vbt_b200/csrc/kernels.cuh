@@ -106,7 +106,7 @@ void launch_decode_dense(const DeviceAsset& a, uint32_t seq, const int* frames, 
 void launch_decode_cache_warp(const DeviceAsset& a, const int* frames, int nframes, float* out, uint64_t stride,
                               int grid, cudaStream_t s);
 int decode_warp_grid();
-// (d) scientific window decode on the tensor cores, frames [t0, t0 + n), n <= 64, cache layout.
+// (d) scientific window decode, frames [t0, t0 + n), n <= 64, cache layout (the exact frames kernel).
 void launch_sci_window(const DeviceAsset& a, int t0, int n, float* out, uint64_t frame_stride, cudaStream_t s);
 // FP64 oracle of a scientific window: stats[0] max |err| (double bits), stats[1] sum err^2
 // (double), stats[2] / stats[3] oracle min / max (order-preserving bits).
