@@ -323,7 +323,7 @@ __device__ LeafEntry walk_sci_leaf(const DeviceAsset& a, uint32_t leaf)
 }
 
 // Page-table compaction of one tile of kWalkTile leaves (one flag per thread): ballot/popc within
-// warps, a serial scan over the tile's warps, and a single-pass decoupled look-back across tiles
+// warps, a serial scan over the tile's warps, and a single-pass decoupled look-back of a warp across tiles
 // (epoch-tagged descriptors, bounded spin).  Writes compact[], active_list[] and, from the last
 // tile, the active count.
 __device__ __forceinline__ void compact_tile(const DeviceAsset& a, uint32_t epoch, uint32_t tile, bool flag,
@@ -337,43 +337,52 @@ __device__ __forceinline__ void compact_tile(const DeviceAsset& a, uint32_t epoc
     const uint32_t in_warp = __popc(bal & ((1u << lane) - 1u));
     if (lane == 0) s_warp[warp] = __popc(bal);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t run = 0;
-        for (int w = 0; w < kWalkThreads / 32; ++w) {
-            const uint32_t c = s_warp[w];
-            s_warp[w] = run;
-            run += c;
-        }
-        // decoupled look-back: descriptor = epoch[63:34] | flag[33:32] (1 aggregate, 2 prefix) | count
+    if (warp == 0) {
+        uint32_t run = 0;   // leaves of the tile, and each warp's first
+        if (lane == 0)
+            for (int w = 0; w < kWalkThreads / 32; ++w) {
+                const uint32_t c = s_warp[w];
+                s_warp[w] = run;
+                run += c;
+            }
+        run = __shfl_sync(0xFFFFFFFFu, run, 0);
+        // decoupled look-back, 32 descriptors at a time (one at a time, the chain of the last tiles was
+        // as long as the table: 32,768 leaves 13 us):
+        // descriptor = epoch[63:34] | flag[33:32] (1 aggregate, 2 prefix) | count
         cuda::atomic_ref<unsigned long long, cuda::thread_scope_device> self(a.tile_state[tile]);
         const unsigned long long ep = (unsigned long long)(epoch & 0x3FFFFFFFu) << 34;
-        uint32_t excl = 0;
-        if (tile == 0) {
-            self.store(ep | (2ull << 32) | run, cuda::memory_order_release);
-        } else {
-            self.store(ep | (1ull << 32) | run, cuda::memory_order_release);
-            int j = (int)tile - 1;
-            uint32_t spins = 0;
-            while (j >= 0) {
-                cuda::atomic_ref<unsigned long long, cuda::thread_scope_device> st(a.tile_state[j]);
-                const unsigned long long v = st.load(cuda::memory_order_acquire);
-                if ((v >> 34) != (unsigned long long)(epoch & 0x3FFFFFFFu) || ((v >> 32) & 3ull) == 0ull) {
-                    if (++spins > (1u << 22)) {   // bounded wait: report and stop, never hang
+        if (lane == 0) self.store(ep | ((tile == 0 ? 2ull : 1ull) << 32) | run, cuda::memory_order_release);
+        uint32_t excl = 0, spins = 0;
+        for (int j = (int)tile - 1; j >= 0;) {
+            const int at = j - lane;   // before the first tile: a prefix of 0
+            unsigned long long v = ep | (2ull << 32);
+            if (at >= 0) {
+                cuda::atomic_ref<unsigned long long, cuda::thread_scope_device> st(a.tile_state[at]);
+                v = st.load(cuda::memory_order_acquire);
+            }
+            const uint32_t flag = (v >> 34) == (ep >> 34) ? (uint32_t)(v >> 32) & 3u : 0u;
+            const unsigned prefix = __ballot_sync(0xFFFFFFFFu, flag == 2u), open = __ballot_sync(0xFFFFFFFFu, flag == 0u);
+            const int last = prefix ? __ffs((int)prefix) - 1 : 31;   // the nearest prefix, or the whole window
+            if (open & (0xFFFFFFFFu >> (31 - last))) {   // a descriptor up to it is not there yet
+                if (++spins > (1u << 22)) {   // bounded wait: report and stop, never hang
+                    if (lane == 0) {
                         atomicOr(a.counters + 1, 1u);
                         record_error(a.err, leaf0, kErrWaitTimeout);
-                        break;
                     }
-                    __nanosleep(64);
-                    continue;
+                    break;
                 }
-                excl += (uint32_t)(v & 0xFFFFFFFFull);
-                if (((v >> 32) & 3ull) == 2ull) break;
-                --j;
+                __nanosleep(32);
+                continue;
             }
-            self.store(ep | (2ull << 32) | (excl + run), cuda::memory_order_release);
+            excl += __reduce_add_sync(0xFFFFFFFFu, lane <= last ? (uint32_t)(v & 0xFFFFFFFFull) : 0u);
+            if (prefix) break;
+            j -= 32;
         }
-        s_base = excl;
-        if (leaf0 + kWalkTile >= L) a.counters[0] = excl + run;   // last tile: total active count
+        if (lane == 0) {
+            if (tile != 0) self.store(ep | (2ull << 32) | (excl + run), cuda::memory_order_release);
+            s_base = excl;
+            if (leaf0 + kWalkTile >= L) a.counters[0] = excl + run;   // last tile: total active count
+        }
     }
     __syncthreads();
     if (leaf < L) {
@@ -936,44 +945,6 @@ struct FrameList {
     int f[kMaxLaunchFrames];
 };
 
-// Leaf per warp (render-temporal caches): the shape the autotuner weighs against the leaf-per-CTA kernel.
-__global__ void __launch_bounds__(kDecodeWarps * 32, 2) decode_kernel(DeviceAsset a, FrameList fl, float* __restrict__ out,
-                                                                     uint64_t frame_stride)
-{
-    __shared__ __align__(16) float s_ctrl_all[kDecodeWarps][kWarpSlots];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float* s_ctrl = s_ctrl_all[warp];
-    const uint32_t n_items = *(volatile const uint32_t*)a.counters;
-    const uint32_t warps_total = gridDim.x * kDecodeWarps;
-    for (uint32_t item = blockIdx.x * kDecodeWarps + warp; item < n_items; item += warps_total) {
-        const uint32_t leaf = __ldg(a.active_list + item);
-        const LeafEntry e = a.entries[leaf];
-        uint32_t bx, by, bz;
-        int w, h, d;
-        leaf_extent(a.g, leaf, bx, by, bz, w, h, d);
-        const bool empty = (e.header & 3u) == kModeEmpty;
-        const uint32_t st = entry_status(e);
-        if (st != kOk && lane == 0) record_error(a.err, leaf, st);
-        for (int fi = 0; fi < fl.n; ++fi) {
-            if (!empty && st == kOk) rt_decode_controls(a, e, clamp_frame(fl.f[fi], (int)a.g.frames), s_ctrl, lane);
-            __syncwarp();
-            for (int r = lane; r < 64; r += 32) {
-                float v[8];
-                if (empty || st != kOk) {
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) v[i] = 0.0f;
-                } else {
-                    rt_row(a, e, s_ctrl, w, h, d, r & 7, r >> 3, v);
-                }
-                float4* dst = reinterpret_cast<float4*>(out + (uint64_t)fi * frame_stride + (uint64_t)item * 512u + r * 8);
-                dst[0] = make_float4(v[0], v[1], v[2], v[3]);
-                dst[1] = make_float4(v[4], v[5], v[6], v[7]);
-            }
-            __syncwarp();
-        }
-    }
-}
-
 }  // namespace vbtb
 #include "sci_frames.cuh"
 namespace vbtb {
@@ -981,20 +952,26 @@ namespace vbtb {
 // Render-temporal decode kernel (TMA-staged leaf, one CTA per leaf): rt_kernel_leaf.cuh
 }  // namespace vbtb
 #include "rt_kernel_leaf.cuh"
+#include "rt_frames.cuh"
 namespace vbtb {
 
-static int default_grid()
+// CTAs that fill the device once at `per` per SM.
+static int wave(int per)
 {
-    static int g = 0;
-    if (!g) {
-        int dev = 0, sms = 0, per = 0;
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, decode_kernel, kDecodeWarps * 32, 0);
-        g = sms * (per > 0 ? per : 1);
     }
-    return g;
+    return (sms > 0 ? sms : 1) * (per > 0 ? per : 1);
 }
+
+// Up to this many frames a launch reads the keys of each frame from the payload (rt_frames.cuh); more
+// are streamed from whole leaves in shared memory (rt_kernel_leaf.cuh).  Caches on a B200, read against
+// streamed: 6 frames of a 128 x 128 x 192 fire 89 / 112 us, of a 256^3 plume 81 / 94, of a 128^3 level
+// set 63 / 101; 8 frames 116 / 124, 107 / 102, 79 / 109; 16 frames 216 / 181, 194 / 141, 136 / 159.
+constexpr int kFewFrames = 6;
 
 void launch_decode_cache(const DeviceAsset& a, uint32_t seq, const int* frames, int nframes, float* out,
                          uint64_t stride, int grid, cudaStream_t s)
@@ -1004,6 +981,8 @@ void launch_decode_cache(const DeviceAsset& a, uint32_t seq, const int* frames, 
     for (int i = 0; i < nframes; ++i) fl.f[i] = frames[i];
     if (a.g.profile == 2u)
         launch_sci_frames<false>(a, fl, out, stride, grid, s);
+    else if (nframes <= kFewFrames && grid == 0)
+        launch_rt_frames<false>(a, fl, out, stride, 0, s);
     else
         launch_rt_leaf(a, seq, fl, out, stride, grid, false, s);
 }
@@ -1015,24 +994,26 @@ void launch_decode_cache(const DeviceAsset& a, uint32_t seq, const int* frames, 
 // blends with mix(), which can differ in the last bit).  One CTA per active leaf at a time.
 constexpr uint32_t kControlCacheStride = 576u;
 
-__global__ void __launch_bounds__(256) control_cache_kernel(DeviceAsset a, FrameList fl, float* __restrict__ out,
+constexpr int kControlCtas = 5;   // 40 warps of at most 48 registers: the control reads are latency
+__global__ void __launch_bounds__(256, kControlCtas) control_cache_kernel(DeviceAsset a, FrameList fl, float* __restrict__ out,
                                                             uint64_t frame_stride)
 {
     const uint32_t n_leaves = *(volatile const uint32_t*)a.counters;
     const int total = (int)a.g.frames;
-    const uint32_t* __restrict__ pw = a.payload;
     for (uint32_t rank = blockIdx.x; rank < n_leaves; rank += gridDim.x) {
         const uint32_t leaf = __ldg(a.active_list + rank);
         const LeafEntry e = a.entries[leaf];
         const uint32_t st = entry_status(e);
         const bool ok = st == kOk && (e.header & 3u) != kModeEmpty;
         if (st != kOk && threadIdx.x == 0) record_error(a.err, leaf, st);
-        const uint64_t base = 4ull * e.word_off;
+        const uint32_t* __restrict__ lw = a.payload + e.word_off;
         const uint32_t cres = (e.header >> 6) & 7u, fres = (e.header >> 9) & 7u;
         const bool fine = (e.info & kFlagFine) != 0u, shell = (e.info & kFlagShell) != 0u;
-        const StreamRef cs{base + 8u, cres * cres * cres, 8u, e.kf & 0xFFFFu, (e.header >> 2) & 3u};
-        const StreamRef fs{base + 8u + e.coarse_bytes, fres * fres * fres, 8u, e.kf >> 16, (e.header >> 4) & 3u};
-        const StreamRef ss{base + e.shell_off, entry_shell_active(e), 4u, e.kf >> 16, (e.header >> 4) & 3u};
+        const uint32_t ccodec = (e.header >> 2) & 3u, fcodec = (e.header >> 4) & 3u;
+        const bool sorted = (e.info & kFlagSorted) != 0u;
+        const LeafStream cs{lw, 8u, cres * cres * cres, 8u, e.kf & 0xFFFFu};
+        const LeafStream fs{lw, 8u + e.coarse_bytes, fres * fres * fres, 8u, e.kf >> 16};
+        const LeafStream ss{lw, e.shell_off, entry_shell_active(e), 4u, e.kf >> 16};
         for (int j = 0; j < fl.n; ++j) {
             const int t = clamp_frame(fl.f[j], total);
             const uint32_t b8 = time_bin(t, 8u, total), b4 = time_bin(t, 4u, total);
@@ -1041,11 +1022,11 @@ __global__ void __launch_bounds__(256) control_cache_kernel(DeviceAsset a, Frame
                 float v = 0.0f;
                 if (ok) {
                     if (slot < 64u) {
-                        if (slot < cs.controls) v = decode_control(pw, cs, slot, t, b8);
+                        if (slot < cs.controls) v = control_at(cs, ccodec, slot, t, b8, sorted);
                     } else {
                         const uint32_t ci = slot - 64u;
-                        if (fine && ci < fs.controls) v = decode_control(pw, fs, ci, t, b8);
-                        else if (shell && ci < ss.controls) v = decode_control(pw, ss, ci, t, b4);
+                        if (fine && ci < fs.controls) v = control_at(fs, fcodec, ci, t, b8, sorted);
+                        else if (shell && ci < ss.controls) v = control_at(ss, fcodec, ci, t, b4, sorted);
                     }
                 }
                 o[slot] = v;
@@ -1060,7 +1041,7 @@ void launch_control_cache(const DeviceAsset& a, const int* frames, int nframes, 
     FrameList fl{};
     fl.n = nframes;
     for (int i = 0; i < nframes; ++i) fl.f[i] = frames[i];
-    control_cache_kernel<<<default_grid(), 256, 0, s>>>(a, fl, out, stride);
+    control_cache_kernel<<<wave(kControlCtas), 256, 0, s>>>(a, fl, out, stride);
 }
 
 void launch_decode_dense(const DeviceAsset& a, uint32_t seq, const int* frames, int nframes, float* out, int grid,
@@ -1072,6 +1053,8 @@ void launch_decode_dense(const DeviceAsset& a, uint32_t seq, const int* frames, 
     const uint64_t stride = (uint64_t)a.g.width * a.g.height * a.g.depth;
     if (a.g.profile == 2u)
         launch_sci_frames<true>(a, fl, out, stride, grid, s);
+    else if (nframes <= kFewFrames && grid == 0)
+        launch_rt_frames<true>(a, fl, out, stride, 0, s);
     else
         launch_rt_leaf(a, seq, fl, out, stride, grid, true, s);
 }
@@ -1085,10 +1068,10 @@ void launch_decode_cache_warp(const DeviceAsset& a, const int* frames, int nfram
     fl.n = nframes;
     for (int i = 0; i < nframes; ++i) fl.f[i] = frames[i];
     if (a.g.profile == 2u) launch_sci_frames<false>(a, fl, out, stride, grid, s);
-    else decode_kernel<<<grid > 0 ? grid : default_grid(), kDecodeWarps * 32, 0, s>>>(a, fl, out, stride);
+    else launch_rt_frames<false>(a, fl, out, stride, grid, s);
 }
 
-int decode_warp_grid() { return default_grid(); }
+int decode_warp_grid() { return wave(kRtCtas); }
 
 // Plain per-leaf launch: grid = the whole leaf grid, one 64-thread CTA per leaf (EMPTY leaves
 // return at once), controls decoded by both warps' lanes, one frame.  This is the reference
@@ -1136,56 +1119,70 @@ void launch_decode_cache_plain(const DeviceAsset& a, int frame, float* out, cuda
 #include "point_query.cuh"
 namespace vbtb {
 
-// Z-slice over [t0, t1): one warp per (leaf of the z layer, frame); lanes 0..7 produce rows.
-__global__ void __launch_bounds__(kDecodeWarps * 32) query_slice_kernel(DeviceAsset a, uint32_t z, int t0, int t1,
-                                                                        float* __restrict__ out)
+// Rows of one leaf of a z layer at frame t, by a warp: `dst` is the layer's row 0 at the leaf's first
+// voxel (zeros for EMPTY leaves, failed ones and frames of a scientific asset out of range).
+__device__ __forceinline__ void slice_tile(const DeviceAsset& a, uint32_t leaf, uint32_t z, int t, float* __restrict__ dst,
+                                           float* __restrict__ sm, const float4* w16, unsigned long long* err)
 {
-    __shared__ __align__(16) float s_ctrl_all[kDecodeWarps][kWarpSlots];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float* s_ctrl = s_ctrl_all[warp];
-    const uint32_t bz = min(a.g.lcz - 1u, z >> 3);
+    const int lane = threadIdx.x & 31;
+    const LeafEntry e = a.entries[leaf];
+    uint32_t bx, by, bz;
+    int w, h, d;
+    leaf_extent(a.g, leaf, bx, by, bz, w, h, d);
     const int lz = (int)(z - bz * 8u);
+    const uint32_t st = entry_status(e);
+    const bool sci = a.g.profile == 2u;
+    if (st != kOk && lane == 0) record_error(err, leaf, st);
+    auto put = [&](int ly, int lx0, float4 v) {
+        if (ly < h) store_row_quad(dst + (uint64_t)((uint32_t)ly) * a.g.width + (uint32_t)lx0, lx0, w, v);
+    };
+    if (st != kOk || lz >= d || (sci ? (uint32_t)t >= a.g.frames : (e.header & 3u) == kModeEmpty)) {
+        if (lane < 16) put(lane >> 1, 4 * (lane & 1), make_float4(0.f, 0.f, 0.f, 0.f));
+        return;
+    }
+    if (!sci) {
+        rt_leaf_layer(a, e, clamp_frame(t, (int)a.g.frames), w, h, d, lz, sm, w16, put);
+        return;
+    }
+    bool oob = false;
+    sci_decode_controls(a, e, (uint32_t)t, sm, lane, oob);
+    __syncwarp();
+    if (lane < 8) {
+        float v[8];
+        sci_row(a, e, sm, (uint32_t)t, w, h, d, lane, lz, v, oob);
+        put(lane, 0, make_float4(v[0], v[1], v[2], v[3]));
+        put(lane, 4, make_float4(v[4], v[5], v[6], v[7]));
+    }
+    if (__any_sync(0xFFFFFFFFu, oob) && lane == 0) record_error(err, leaf, kErrDecodeOob);
+    __syncwarp();
+}
+
+// Z-slice over [t0, t1): one warp per (leaf of the z layer, frame).
+constexpr int kSliceCtas = 6;
+static_assert(kRtWarpFloats >= 64 + 16 * 64, "room for the scientific controls and residual grids");
+__global__ void __launch_bounds__(kRtWarps * 32, kSliceCtas) query_slice_kernel(DeviceAsset a, uint32_t z, int t0, int t1,
+                                                                               float* __restrict__ out)
+{
+    __shared__ __align__(16) float s_all[kRtWarps][kRtWarpFloats];
+    __shared__ float4 s_w16[48];
+    fill_axis_rows(s_w16);
+    const int warp = threadIdx.x >> 5;
+    const uint32_t bz = min(a.g.lcz - 1u, z >> 3);
     const uint32_t layer = a.g.lcx * a.g.lcy;
     const uint32_t n_items = layer * (uint32_t)(t1 - t0);
-    for (uint32_t item = blockIdx.x * kDecodeWarps + warp; item < n_items; item += gridDim.x * kDecodeWarps) {
-        const uint32_t li = item % layer;
-        const int t = t0 + (int)(item / layer);
-        const uint32_t leaf = bz * layer + li;
-        const LeafEntry e = a.entries[leaf];
-        uint32_t bx, by, bzz;
-        int w, h, d;
-        leaf_extent(a.g, leaf, bx, by, bzz, w, h, d);
-        const uint32_t st = entry_status(e);
-        const bool empty = a.g.profile != 2u && (e.header & 3u) == kModeEmpty;
-        bool oob = false;
-        const bool in_range = lz < d && (a.g.profile != 2u || (uint32_t)t < a.g.frames);
-        if (st != kOk && lane == 0) record_error(a.err, leaf, st);
-        if (in_range && !empty && st == kOk) {
-            if (a.g.profile == 2u) sci_decode_controls(a, e, (uint32_t)t, s_ctrl, lane, oob);
-            else rt_decode_controls(a, e, clamp_frame(t, (int)a.g.frames), s_ctrl, lane);
-        }
-        __syncwarp();
-        if (lane < 8 && lane < h) {
-            float v[8];
-            if (!in_range || empty || st != kOk) {
-                for (int i = 0; i < 8; ++i) v[i] = 0.0f;
-            } else if (a.g.profile == 2u) {
-                sci_row(a, e, s_ctrl, (uint32_t)t, w, h, d, lane, lz, v, oob);
-            } else {
-                rt_row(a, e, s_ctrl, w, h, d, lane, lz, v);
-            }
-            float* dst = out + (uint64_t)(t - t0) * a.g.width * a.g.height + (uint64_t)(by * 8 + lane) * a.g.width + bx * 8;
-            for (int i = 0; i < w; ++i) dst[i] = v[i];
-        }
-        if (__any_sync(0xFFFFFFFFu, oob) && lane == 0) record_error(a.err, leaf, kErrDecodeOob);
-        __syncwarp();
+    for (uint32_t item = blockIdx.x * kRtWarps + warp; item < n_items; item += gridDim.x * kRtWarps) {
+        const uint32_t li = item % layer, f = item / layer;
+        const uint64_t at = ((uint64_t)f * a.g.height + li / a.g.lcx * 8u) * a.g.width + li % a.g.lcx * 8u;
+        slice_tile(a, bz * layer + li, z, t0 + (int)f, out + at, s_all[warp], s_w16, a.err);
     }
 }
 
 void launch_query_slice(const DeviceAsset& a, uint32_t z, int t0, int t1, float* out, cudaStream_t s)
 {
     if (t1 <= t0) return;
-    query_slice_kernel<<<default_grid(), kDecodeWarps * 32, 0, s>>>(a, z, t0, t1, out);
+    const uint64_t items = (uint64_t)a.g.lcx * a.g.lcy * (uint64_t)(t1 - t0), ctas = (items + kRtWarps - 1) / kRtWarps;
+    const uint64_t most = (uint64_t)wave(kSliceCtas);
+    query_slice_kernel<<<(unsigned)(ctas < most ? ctas : most), kRtWarps * 32, 0, s>>>(a, z, t0, t1, out);
 }
 
 }  // namespace vbtb

@@ -178,54 +178,105 @@ struct LeafStream {
     uint32_t base, controls, bins, kf;
 };
 
-// Control c of an FP16 stream whose key frames strictly increase, at clamped frame `frame`: the value
+// Controls of FP16 streams whose key frames strictly increase, at a clamped frame: the value
 // decode_control's search gives (for such keys the canonical one: the first key's value before it,
 // the last key's after it, the key's on an exact hit, else the lerp of the pair around the frame;
 // see the head of rt_staged.cuh).  Four keys (12 bytes from the hinted one on) are taken at a time
 // as independent word reads and the pair is selected in registers: a time bin rarely spans more, so
 // a control is two dependent steps (descriptor and hint, keys) where the search's halving makes
-// four to seven.  The payload's 16-byte tail padding covers the words past the last key.
+// four to seven.  The payload's 16-byte tail padding covers the words past the last key.  The steps
+// are apart so that a lane can have the reads of several controls in flight.
+struct KeyWindow {
+    uint32_t kb, kc, lo;      // byte offset of the control's first key, its keys, the window's first
+    uint32_t x0, x1, x2, x3;  // words from the window's first byte on
+};
+
+__device__ __forceinline__ void key_window(const uint32_t* __restrict__ lw, KeyWindow& k)
+{
+    const uint32_t* w = lw + ((k.kb + 3u * k.lo) >> 2);
+    k.x0 = __ldg(w);
+    k.x1 = __ldg(w + 1);
+    k.x2 = __ldg(w + 2);
+    k.x3 = __ldg(w + 3);
+}
+
+// The window a control's descriptor and hint word name; kc 0 where it decodes to 0 (see decode_control).
+__device__ __forceinline__ KeyWindow key_start(const LeafStream& s, uint32_t desc, uint32_t hints, uint32_t bin)
+{
+    const uint32_t kc = (desc >> 16) & 0xFFu, ks = desc & 0xFFFFu, hb = (hints >> ((bin & 3u) * 8u)) & 0xFFu;
+    KeyWindow k{};
+    k.kc = ks + kc > s.kf ? 0u : kc;
+    k.kb = s.base + s.controls * 4u + align4(s.controls * s.bins) + 3u * ks;
+    k.lo = hb + 1u < kc ? hb : kc - 1u;
+    return k;
+}
+
+// a / b for 0 <= a <= b <= 255, correctly rounded: the product with the approximate reciprocal and one
+// fused remainder step (P. Markstein, IBM J. Res. Dev. 34(1), 1990).  A quotient of such integers is at
+// least 2^-9 of a unit in the last place away from a rounding boundary, far more than the reciprocal's
+// error moves the corrected one (checked for every pair with reciprocals off by up to two units).
+__device__ __forceinline__ float div_u8_rn(float a, float b)
+{
+    float y;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(b));
+    const float q = __fmul_rn(a, y);
+    return __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
+}
+
+// An integer below 2^23 as a float, without the conversion unit.
+__device__ __forceinline__ float small_to_float(uint32_t x)
+{
+    return __fsub_rn(__uint_as_float(x | 0x4B000000u), 8388608.0f);
+}
+
+// The value at `frame`, moving the window where the pair lies elsewhere.  PLAIN: no key is a NaN
+// (kFlagHalfPlain).  About 60 instructions, of which a move repeats a quarter.
+template <bool PLAIN>
+__device__ __forceinline__ float key_value_at(const uint32_t* __restrict__ lw, KeyWindow k, int frame)
+{
+    if (k.kc == 0u) return 0.0f;
+    uint32_t a0, a1, a2, left;
+    for (;; key_window(lw, k)) {
+        const uint32_t sh = ((k.kb + 3u * k.lo) & 3u) * 8u;
+        a0 = __funnelshift_r(k.x0, k.x1, sh);
+        a1 = __funnelshift_r(k.x1, k.x2, sh);
+        a2 = __funnelshift_r(k.x2, k.x3, sh);
+        left = k.kc - k.lo;   // keys from lo on
+        if ((int)(a0 & 0xFFu) > frame && k.lo != 0u) k.lo = 0u;                        // the hint overshot
+        else if (left > 4u && (int)((a2 >> 8) & 0xFFu) <= frame) k.lo += 3u;   // the pair may lie further on
+        else break;
+    }
+    // keys 0..3 of the window: frame in the low byte, value above it; p1..p3: key i is there and not past the frame
+    const uint32_t k1 = __byte_perm(a0, a1, 0x0543), k2 = __byte_perm(a1, a2, 0x0432), k3 = a2 >> 8;
+    const bool p1 = left > 1u && (int)(a0 >> 24) <= frame, p2 = left > 2u && (int)(k2 & 0xFFu) <= frame,
+               p3 = left > 3u && (int)(k3 & 0xFFu) <= frame;
+    const uint32_t lower = p3 ? k3 : p2 ? k2 : p1 ? k1 : a0, upper = p2 ? k3 : p1 ? k2 : k1;
+    const bool end = left == (p3 ? 4u : p2 ? 3u : p1 ? 2u : 1u);   // no key after the lower one
+    const int ahead = frame - (int)(lower & 0xFFu);                // below 0: before the first key
+    auto value = [](uint32_t key) {
+        const uint32_t h = (key >> 8) & 0xFFFFu;
+        return PLAIN ? __half2float(__ushort_as_half((unsigned short)h)) : half_to_float_exact(h);
+    };
+    const float vp = value(lower);
+    if (end || ahead <= 0) return vp;   // past the last key, an exact hit, before the first key
+    const float vn = value(upper);
+    const float alpha = div_u8_rn(small_to_float((uint32_t)ahead), small_to_float((upper & 0xFFu) - (lower & 0xFFu)));
+    return __fadd_rn(vp, __fmul_rn(alpha, __fsub_rn(vn, vp)));
+}
+
+__device__ __forceinline__ uint32_t hint_word(const LeafStream& s, uint32_t c, uint32_t bin)
+{
+    return __ldg(s.w + ((s.base + 4u * s.controls + c * s.bins + bin) >> 2));
+}
+
+template <bool PLAIN>
 __device__ __forceinline__ float control_sorted(const LeafStream& s, uint32_t c, int frame, uint32_t bin)
 {
     const uint32_t desc = __ldg(s.w + (s.base >> 2) + c);
-    const uint32_t w0 = __ldg(s.w + ((s.base + 4u * s.controls + c * s.bins + bin) >> 2));
-    const uint32_t kc = (desc >> 16) & 0xFFu, ks = desc & 0xFFFFu;
-    if (kc == 0u || ks + kc > s.kf) return 0.0f;   // see decode_control
-    const uint32_t kb = s.base + s.controls * 4u + align4(s.controls * s.bins) + 3u * ks;
-    const uint32_t hb = (w0 >> ((bin & 3u) * 8u)) & 0xFFu;
-    uint32_t lo = hb < kc - 1u ? hb : kc - 1u;
-    for (;;) {
-        const uint32_t b = kb + 3u * lo;
-        const uint32_t* w = s.w + (b >> 2);
-        const uint32_t sh = (b & 3u) * 8u;
-        const uint32_t x0 = __ldg(w), x1 = __ldg(w + 1), x2 = __ldg(w + 2), x3 = __ldg(w + 3);
-        const uint32_t a0 = __funnelshift_r(x0, x1, sh), a1 = __funnelshift_r(x1, x2, sh),
-                       a2 = __funnelshift_r(x2, x3, sh);
-        const uint32_t left = kc - lo;   // keys from lo on
-        const int f0 = (int)(a0 & 0xFFu), f1 = (int)(a0 >> 24), f2 = (int)((a1 >> 16) & 0xFFu),
-                  f3 = (int)((a2 >> 8) & 0xFFu);
-        const uint32_t h0 = (a0 >> 8) & 0xFFFFu, h1 = a1 & 0xFFFFu, h2 = __byte_perm(a1, a2, 0x0043) & 0xFFFFu,
-                       h3 = a2 >> 16;
-        if (f0 > frame) {
-            if (lo == 0u) return half_to_float_exact(h0);
-            lo = 0u;   // the hint overshot
-            continue;
-        }
-        const bool p1 = left > 1u && f1 <= frame, p2 = left > 2u && p1 && f2 <= frame,
-                   p3 = left > 3u && p2 && f3 <= frame;
-        if (p3 && left > 4u) {   // the pair may lie further on
-            lo += 3u;
-            continue;
-        }
-        const int fp = p3 ? f3 : p2 ? f2 : p1 ? f1 : f0;
-        const float vp = half_to_float_exact(p3 ? h3 : p2 ? h2 : p1 ? h1 : h0);
-        const uint32_t at = p3 ? 3u : p2 ? 2u : p1 ? 1u : 0u;
-        if (fp == frame || at + 1u == left) return vp;   // an exact hit, or past the last key
-        const int fn = p2 ? f3 : p1 ? f2 : f1;
-        const float vn = half_to_float_exact(p2 ? h3 : p1 ? h2 : h1);
-        const float alpha = __fdiv_rn((float)(frame - fp), (float)(fn - fp));
-        return __fadd_rn(vp, __fmul_rn(alpha, __fsub_rn(vn, vp)));
-    }
+    KeyWindow k = key_start(s, desc, hint_word(s, c, bin), bin);
+    if (k.kc == 0u) return 0.0f;
+    key_window(s.w, k);
+    return key_value_at<PLAIN>(s.w, k, frame);
 }
 
 // The reference's search as a call of its own (leaves with unordered keys or FP32 keys).
@@ -239,7 +290,7 @@ __device__ __noinline__ static float control_searched(const uint32_t* w, uint32_
 __device__ __forceinline__ float control_at(const LeafStream& s, uint32_t codec, uint32_t c, int frame, uint32_t bin,
                                             bool sorted)
 {
-    if (sorted && codec != 1u) return control_sorted(s, c, frame, bin);
+    if (sorted && codec != 1u) return control_sorted<false>(s, c, frame, bin);
     return control_searched(s.w, s.base, s.controls, s.bins, s.kf, codec, c, frame, bin);
 }
 

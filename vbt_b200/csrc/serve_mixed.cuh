@@ -6,10 +6,9 @@
 //
 // The requests form a table (MixedReq, in device memory) with a running count of tiles.  A tile is
 // one warp's piece of work:
-//   slice   one (leaf of the z layer, frame): the leaf's controls at the frame, then its rows of
-//           the layer -- the body of query_slice_kernel;
-//   frames  one (leaf, frame) of a dense frame: controls, then all 64 rows of the leaf (zeros for
-//           an EMPTY leaf) -- the body of the warp-per-leaf decode_kernel<DENSE>.
+//   slice   one (leaf of the z layer, frame): slice_tile, as query_slice_kernel;
+//   frames  one (leaf, frame) of a dense frame (zeros for an EMPTY leaf): rt_leaf_frame, as
+//           rt_frames_kernel, or the scientific per-frame functions.
 // Warps take tiles kTileGrab at a time from a work counter (zeroed before the launch), so the
 // tiles of large and small requests spread over the GPU as they come.  Each request has its own
 // result array and error word; the values are those of the per-request kernels, bit for bit.
@@ -25,92 +24,46 @@ __host__ __device__ __forceinline__ uint64_t mixed_tiles(const MixedReq& r, cons
     return r.kind == kMixedSlice ? (uint64_t)g.lcx * g.lcy * (uint64_t)(r.t1 - r.t0) : (uint64_t)g.leaf_count * r.n;
 }
 
-// Slice tile: rows of leaf `li` of the z layer at frame t into the request's [t - t0][y][x] output.
-__device__ __forceinline__ void mixed_slice_tile(const DeviceAsset& a, const MixedReq& r, uint32_t li, int t,
-                                                 float* __restrict__ s_ctrl, unsigned long long* err, int lane)
-{
-    const uint32_t bz = min(a.g.lcz - 1u, r.a0 >> 3);
-    const int lz = (int)(r.a0 - bz * 8u);
-    const uint32_t leaf = bz * a.g.lcx * a.g.lcy + li;
-    const LeafEntry e = a.entries[leaf];
-    uint32_t bx, by, bzz;
-    int w, h, d;
-    leaf_extent(a.g, leaf, bx, by, bzz, w, h, d);
-    const uint32_t st = entry_status(e);
-    const bool sci = a.g.profile == 2u;
-    const bool empty = !sci && (e.header & 3u) == kModeEmpty;
-    bool oob = false;
-    const bool in_range = lz < d && (!sci || (uint32_t)t < a.g.frames);
-    if (st != kOk && lane == 0) record_error(err, leaf, st);
-    if (in_range && !empty && st == kOk) {
-        if (sci) sci_decode_controls(a, e, (uint32_t)t, s_ctrl, lane, oob);
-        else rt_decode_controls(a, e, clamp_frame(t, (int)a.g.frames), s_ctrl, lane);
-    }
-    __syncwarp();
-    if (lane < 8 && lane < h) {
-        float v[8];
-        if (!in_range || empty || st != kOk) {
-            for (int i = 0; i < 8; ++i) v[i] = 0.0f;
-        } else if (sci) {
-            sci_row(a, e, s_ctrl, (uint32_t)t, w, h, d, lane, lz, v, oob);
-        } else {
-            rt_row(a, e, s_ctrl, w, h, d, lane, lz, v);
-        }
-        float* out = reinterpret_cast<float*>(r.out);
-        float* dst = out + (uint64_t)(t - r.t0) * a.g.width * a.g.height + (uint64_t)(by * 8 + lane) * a.g.width + bx * 8;
-        for (int i = 0; i < w; ++i) dst[i] = v[i];
-    }
-    if (__any_sync(0xFFFFFFFFu, oob) && lane == 0) record_error(err, leaf, kErrDecodeOob);
-    __syncwarp();
-}
-
-// Frame tile: all voxels of `leaf` at frame index `fr` (as given) into the dense frame `frame_out`.
+// Frame tile: all voxels of `leaf` at frame index `fr` (as given) into the dense frame `fb`.
 __device__ __forceinline__ void mixed_frame_tile(const DeviceAsset& a, uint32_t leaf, int fr, float* __restrict__ fb,
-                                                 float* __restrict__ s_ctrl, unsigned long long* err, int lane)
+                                                 float* __restrict__ sm, const float4* w16, unsigned long long* err)
 {
+    const int lane = threadIdx.x & 31;
     const LeafEntry e = a.entries[leaf];
     uint32_t bx, by, bz;
     int w, h, d;
     leaf_extent(a.g, leaf, bx, by, bz, w, h, d);
     const bool sci = a.g.profile == 2u;
-    const bool empty = !sci && (e.header & 3u) == kModeEmpty;
     const uint32_t st = entry_status(e);
     if (st != kOk && lane == 0) record_error(err, leaf, st);
-    const bool scatter = sci && st == kOk && (e.header & 3u) == 1u && (e.info & kFlagSorted) != 0u;
-    bool oob = false;
-    if (!empty && st == kOk) {
-        if (sci) sci_decode_controls(a, e, (uint32_t)fr, s_ctrl, lane, oob);
-        else rt_decode_controls(a, e, clamp_frame(fr, (int)a.g.frames), s_ctrl, lane);
+    float* const dst = fb + ((uint64_t)(bz * 8u) * a.g.height + by * 8u) * a.g.width + bx * 8u;
+    auto put = [&](int ly, int lz, int lx0, float4 v) {
+        if (ly < h && lz < d)
+            store_row_quad(dst + ((uint64_t)((uint32_t)lz) * a.g.height + (uint32_t)ly) * a.g.width + (uint32_t)lx0, lx0, w, v);
+    };
+    if (st != kOk || (!sci && (e.header & 3u) == kModeEmpty)) {
+        for (int r = lane; r < 128; r += 32) put((r >> 1) & 7, r >> 4, 4 * (r & 1), make_float4(0.f, 0.f, 0.f, 0.f));
+        return;
     }
+    if (!sci) {
+        rt_leaf_frame(a, e, clamp_frame(fr, (int)a.g.frames), w, h, d, sm, w16, put);
+        return;
+    }
+    const bool scatter = (e.header & 3u) == 1u && (e.info & kFlagSorted) != 0u;
+    bool oob = false;
+    sci_decode_controls(a, e, (uint32_t)fr, sm, lane, oob);
     __syncwarp();
-    for (int rr = lane; rr < 64; rr += 32) {
-        const int ly = rr & 7, lz = rr >> 3;
+    for (int r = lane; r < 64; r += 32) {
         float v[8];
-        if (empty || st != kOk) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = 0.0f;
-        } else if (sci) {
-            sci_row(a, e, s_ctrl, (uint32_t)fr, w, h, d, ly, lz, v, oob, scatter);
-        } else {
-            rt_row(a, e, s_ctrl, w, h, d, ly, lz, v);
-        }
-        if (ly < h && lz < d) {
-            float* dst = fb + ((uint64_t)(bz * 8 + lz) * a.g.height + (by * 8 + ly)) * a.g.width + bx * 8;
-            if (w == 8 && (((uintptr_t)dst) & 15u) == 0u) {
-                reinterpret_cast<float4*>(dst)[0] = make_float4(v[0], v[1], v[2], v[3]);
-                reinterpret_cast<float4*>(dst)[1] = make_float4(v[4], v[5], v[6], v[7]);
-            } else {
-                for (int i = 0; i < w; ++i) dst[i] = v[i];
-            }
-        }
+        sci_row(a, e, sm, (uint32_t)fr, w, h, d, r & 7, r >> 3, v, oob, scatter);
+        put(r & 7, r >> 3, 0, make_float4(v[0], v[1], v[2], v[3]));
+        put(r & 7, r >> 3, 4, make_float4(v[4], v[5], v[6], v[7]));
     }
     if (scatter && (uint32_t)fr < a.g.frames) {
         __syncwarp();   // the rows written by the other lanes are visible
         sci_scatter_frame(a, e, (uint32_t)fr, w, h, d, lane,
                           [&](uint32_t li) {
-                              return fb + ((uint64_t)(bz * 8 + (li >> 6)) * a.g.height + (by * 8 + ((li >> 3) & 7u))) *
-                                              a.g.width +
-                                          bx * 8 + (li & 7u);
+                              return dst + ((uint64_t)(li >> 6) * a.g.height + ((li >> 3) & 7u)) * a.g.width + (li & 7u);
                           },
                           oob);
     }
@@ -120,18 +73,19 @@ __device__ __forceinline__ void mixed_frame_tile(const DeviceAsset& a, uint32_t 
 
 constexpr int kMixedWarps = 8;
 
-__global__ void __launch_bounds__(kMixedWarps * 32) serve_mixed_kernel(const DeviceAsset* __restrict__ assets,
+__global__ void __launch_bounds__(kMixedWarps * 32, 3) serve_mixed_kernel(const DeviceAsset* __restrict__ assets,
                                                                        const MixedReq* __restrict__ reqs, uint32_t k,
                                                                        uint64_t n_tiles, unsigned long long* counter,
                                                                        unsigned long long* errs)
 {
-    __shared__ __align__(16) float s_ctrl_all[kMixedWarps][kWarpSlots];
+    __shared__ __align__(16) float s_all[kMixedWarps][kRtWarpFloats];
+    __shared__ float4 s_w16[48];
     __shared__ uint64_t s_first[kMaxMixedReqs + 1];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (uint32_t i = (uint32_t)tid; i < k; i += blockDim.x) s_first[i] = reqs[i].first;
     if (tid == 0) s_first[k] = n_tiles;
-    __syncthreads();
-    float* s_ctrl = s_ctrl_all[warp];
+    fill_axis_rows(s_w16);   // and the table of first tiles is complete
+    float* sm = s_all[warp];
     for (;;) {
         unsigned long long base = 0;
         if (lane == 0) base = atomicAdd(counter, (unsigned long long)kTileGrab);
@@ -152,13 +106,17 @@ __global__ void __launch_bounds__(kMixedWarps * 32) serve_mixed_kernel(const Dev
             unsigned long long* err = errs + lo;
             if (rq.kind == kMixedSlice) {
                 const uint32_t layer = a.g.lcx * a.g.lcy;
-                mixed_slice_tile(a, rq, (uint32_t)(u % layer), rq.t0 + (int)(u / layer), s_ctrl, err, lane);
+                const uint32_t li = (uint32_t)(u % layer), f = (uint32_t)(u / layer);
+                const uint32_t bz = min(a.g.lcz - 1u, rq.a0 >> 3);
+                float* dst = reinterpret_cast<float*>(rq.out) +
+                             ((uint64_t)f * a.g.height + li / a.g.lcx * 8u) * a.g.width + li % a.g.lcx * 8u;
+                slice_tile(a, bz * layer + li, rq.a0, rq.t0 + (int)f, dst, sm, s_w16, err);
             } else {
                 const uint32_t L = a.g.leaf_count;
                 const uint64_t fi = u / L;
                 const int fr = reinterpret_cast<const int*>(rq.in)[fi];
                 float* fb = reinterpret_cast<float*>(rq.out) + fi * ((uint64_t)a.g.width * a.g.height * a.g.depth);
-                mixed_frame_tile(a, (uint32_t)(u % L), fr, fb, s_ctrl, err, lane);
+                mixed_frame_tile(a, (uint32_t)(u % L), fr, fb, sm, s_w16, err);
             }
         }
     }
