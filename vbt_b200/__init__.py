@@ -10,6 +10,7 @@ as raw integer device addresses.
 """
 import ctypes as C
 import os
+import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libvbt_b200.so")
@@ -206,14 +207,15 @@ def _addr(x):
 
 
 def _stream(stream):
+    """cudaStream_t of `stream`: an int, a torch stream, or None for torch's current stream (the legacy
+    default stream in a program that has not used torch on the GPU, where nothing has to be asked)."""
     if stream is None:
-        try:
-            import torch
-            if torch.cuda.is_available():
-                return torch.cuda.current_stream().cuda_stream
-        except Exception:
-            pass
-        return None
+        torch = sys.modules.get("torch")
+        if torch is None or not torch.cuda.is_initialized():
+            return None
+        # the raw handle where torch offers it: building a Stream object takes 3.4 us, a third of a small call
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        return raw(torch.cuda.current_device()) if raw else torch.cuda.current_stream().cuda_stream
     if isinstance(stream, int):
         return stream
     return stream.cuda_stream
