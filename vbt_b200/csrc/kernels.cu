@@ -945,16 +945,6 @@ struct FrameList {
     int f[kMaxLaunchFrames];
 };
 
-}  // namespace vbtb
-#include "sci_frames.cuh"
-namespace vbtb {
-
-// Render-temporal decode kernel (TMA-staged leaf, one CTA per leaf): rt_kernel_leaf.cuh
-}  // namespace vbtb
-#include "rt_kernel_leaf.cuh"
-#include "rt_frames.cuh"
-namespace vbtb {
-
 // CTAs that fill the device once at `per` per SM.
 static int wave(int per)
 {
@@ -966,6 +956,16 @@ static int wave(int per)
     }
     return (sms > 0 ? sms : 1) * (per > 0 ? per : 1);
 }
+
+}  // namespace vbtb
+#include "sci_frames.cuh"
+namespace vbtb {
+
+// Render-temporal decode kernel (TMA-staged leaf, one CTA per leaf): rt_kernel_leaf.cuh
+}  // namespace vbtb
+#include "rt_kernel_leaf.cuh"
+#include "rt_frames.cuh"
+namespace vbtb {
 
 // Up to this many frames a launch reads the keys of each frame from the payload (rt_frames.cuh); more
 // are streamed from whole leaves in shared memory (rt_kernel_leaf.cuh).  Caches on a B200, read against

@@ -45,9 +45,9 @@ constexpr int kMaxLaunchFrames = 128;
 
 // Fixed shared memory of the render decode kernel besides its leaf stage (rt_kernel_leaf.cuh:
 // barrier, frame tables, axis weights, 9 warps x (x-lerp + y-lerp rows), 3072-float controls,
-// reciprocal table, axis weights as 16-byte rows).
+// reciprocal table, lane weights).
 constexpr uint32_t kLeafFixedBytes =
-    16 + 6 * kMaxLaunchFrames + 576 + 9 * 196 * 8 + 9 * 112 * 16 + 3072 * 4 + 256 * 4 + 768;
+    16 + 6 * kMaxLaunchFrames + 576 + 9 * 196 * 8 + 9 * 112 * 16 + 3072 * 4 + 256 * 4 + 5120;
 
 constexpr int kWalkThreads = 256;
 constexpr int kWalkTile = 256;   // leaves per walker CTA (one scan element per thread)

@@ -19,13 +19,14 @@ constexpr int kDecThreads = 32 * kDecWarps;
 constexpr int kLeafCtrlBudget = 3072;   // floats: frames x controls of one batch
 constexpr uint32_t leaf_fixed_bytes(int nw)
 {
-    return 16 + 6 * kMaxLaunchFrames + 576 + nw * 196 * 8 + nw * 112 * 16 + kLeafCtrlBudget * 4 + 256 * 4 + 768;
+    return 16 + 6 * kMaxLaunchFrames + 576 + nw * 196 * 8 + nw * 112 * 16 + kLeafCtrlBudget * 4 + 256 * 4 + 5120;
 }
 constexpr uint32_t kLeafFixed = leaf_fixed_bytes(kLeafWarps);
 constexpr uint32_t kDecFixed = leaf_fixed_bytes(kDecWarps);
 constexpr uint32_t kStagePad = 16;   // readable bytes past the largest staged window
 static_assert(kDecFixed == kLeafFixedBytes, "host stage sizing must match the kernel's shared-memory layout");
 
+struct LaneWeights;
 struct LeafSmem {
     uint64_t* bar;
     int* fr;
@@ -35,7 +36,7 @@ struct LeafSmem {
     float4* y4;      // [warp][112]
     float* ctrl;     // [kLeafCtrlBudget]
     float* rcp;      // [256] RN(1/i)
-    float4* w16;     // [grid][axis][8] {t, 1 - t, i0, i1}: the axis weights as 16-byte rows
+    LaneWeights* lanes;   // [2] the lanes' weights of whole leaves, 4 and 6 controls (rt_leaf_fast.cuh)
     uint8_t* stage;  // leaf window (16-byte aligned), kStagePad bytes of padding after it
 };
 
@@ -53,8 +54,8 @@ __device__ __forceinline__ LeafSmem leaf_layout(uint8_t* dyn)
     s.y4 = reinterpret_cast<float4*>(reinterpret_cast<uint8_t*>(s.x2) + NW * 196 * 8);
     s.ctrl = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(s.y4) + NW * 112 * 16);
     s.rcp = s.ctrl + kLeafCtrlBudget;
-    s.w16 = reinterpret_cast<float4*>(s.rcp + 256);
-    s.stage = reinterpret_cast<uint8_t*>(s.w16 + 48);
+    s.lanes = reinterpret_cast<LaneWeights*>(s.rcp + 256);
+    s.stage = reinterpret_cast<uint8_t*>(s.rcp + 256) + 5120;
     return s;
 }
 
@@ -109,9 +110,8 @@ struct QuadSink {
     uint64_t frame_stride;
     uint32_t li, width, height, bx, by, bz;
     int w, h, d;
-    __device__ __forceinline__ void operator()(int fi, int lane, int i, float4 v) const
+    __device__ __forceinline__ void operator()(int fi, int lz, int ly, int lx0, float4 v) const
     {
-        const int lz = 2 * i + (lane >> 4), ly = (lane >> 1) & 7, lx0 = 4 * (lane & 1);
         if (DENSE) {
             if (ly < h && lz < d) {
                 float* dst = out + (uint64_t)fi * frame_stride +
@@ -124,7 +124,7 @@ struct QuadSink {
                 }
             }
         } else {
-            reinterpret_cast<float4*>(out + (uint64_t)fi * frame_stride + (uint64_t)li * 512u)[lane + 32 * i] = v;
+            *reinterpret_cast<float4*>(out + (uint64_t)fi * frame_stride + (uint64_t)li * 512u + (uint32_t)(64 * lz + 8 * ly + lx0)) = v;
         }
     }
 };
@@ -383,6 +383,7 @@ __global__ void __launch_bounds__(kDecThreads, 2) decode_leaf_kernel(const __gri
         *s_next = first;
     }
     if (tid < 256) s.rcp[tid] = __frcp_rn((float)tid);
+    fill_lane_weights(s.lanes);
     if (tid < fl.n) {
         const int fr = clamp_frame(fl.f[tid], total);
         s.fr[tid] = fr;
@@ -449,7 +450,6 @@ __global__ void __launch_bounds__(kDecThreads, 2) decode_leaf_kernel(const __gri
                 const int ext = axis == 0 ? G.w : (axis == 1 ? G.h : G.d);
                 const AxisWeight aw = g_axis[axis_index(R, ext, p)];
                 s.w[ws][axis][p] = aw;
-                s.w16[tid] = make_float4(aw.t, aw.omt, __int_as_float((int)aw.i0), __int_as_float((int)aw.i1));
             }
             const bool ok = !staged || mbar_wait(s.bar, phase);
             if (__syncthreads_or(!ok)) {   // any thread gave up: the whole CTA stops, together
