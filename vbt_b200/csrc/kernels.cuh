@@ -16,6 +16,7 @@ struct AssetGeom {
     uint32_t stage_bytes;   // shared-memory leaf stage of the render decode kernel (0 = none)
     uint32_t max_window;    // largest 16-byte-aligned window of a non-EMPTY leaf
     uint32_t sparse;        // 1: render-temporal with most leaves EMPTY (the point-query shape)
+    uint32_t mode2;         // 1: some leaf is a Mode2 one (the streaming kernel with its path)
 };
 
 struct DeviceAsset {

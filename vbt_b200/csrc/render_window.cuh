@@ -37,9 +37,9 @@ static_assert(kRwHead % 128u == 0u, "the leaf-kernel layout after the window hea
 
 struct CoefSink {
     float* coef;
-    __device__ __forceinline__ void operator()(int k, int lane, int i, float4 v) const
+    __device__ __forceinline__ void operator()(int k, int lz, int ly, int lx0, float4 v) const
     {
-        reinterpret_cast<float4*>(coef + k * 512)[lane + 32 * i] = v;
+        *reinterpret_cast<float4*>(coef + k * 512 + 64 * lz + 8 * ly + lx0) = v;
     }
 };
 
@@ -258,6 +258,7 @@ __global__ void __launch_bounds__(kLeafThreads, 2) render_window_kernel(DeviceAs
         *s_next = first;
     }
     s.rcp[tid] = __frcp_rn((float)tid);
+    fill_lane_weights(s.lanes);
     win_tc_fence_before();
     __syncthreads();
     win_tc_fence_after();

@@ -70,9 +70,8 @@ namespace vbtb {
 
 template <bool DENSE>
 __device__ __forceinline__ void store_quad(const DeviceAsset& a, const LeafGeom& G, float* __restrict__ out,
-                                           uint64_t frame_stride, int fi, int lane, int i, float4 v)
+                                           uint64_t frame_stride, int fi, int lz, int ly, int lx0, float4 v)
 {
-    const int lz = 2 * i + (lane >> 4), ly = (lane >> 1) & 7, lx0 = 4 * (lane & 1);
     if (DENSE) {
         if (ly < G.h && lz < G.d) {
             float* dst = out + (uint64_t)fi * frame_stride +
@@ -85,7 +84,7 @@ __device__ __forceinline__ void store_quad(const DeviceAsset& a, const LeafGeom&
             }
         }
     } else {
-        reinterpret_cast<float4*>(out + (uint64_t)fi * frame_stride + (uint64_t)G.li * 512u)[lane + 32 * i] = v;
+        *reinterpret_cast<float4*>(out + (uint64_t)fi * frame_stride + (uint64_t)G.li * 512u + (uint32_t)(64 * lz + 8 * ly + lx0)) = v;
     }
 }
 
@@ -96,9 +95,9 @@ struct FrameSink {
     const LeafGeom& G;
     float* __restrict__ out;
     uint64_t frame_stride;
-    __device__ __forceinline__ void operator()(int fi, int lane, int i, float4 v) const
+    __device__ __forceinline__ void operator()(int fi, int lz, int ly, int lx0, float4 v) const
     {
-        store_quad<DENSE>(a, G, out, frame_stride, fi, lane, i, v);
+        store_quad<DENSE>(a, G, out, frame_stride, fi, lz, ly, lx0, v);
     }
 };
 
@@ -130,7 +129,7 @@ struct QuadSink {
 };
 
 // Decode one validated, non-EMPTY leaf for all frames of the launch with word reader `m` and NW
-// warps; each finished quad of 4 voxels goes to `sink(frame index, lane, quad, values)`.  Frame
+// warps; each finished quad of 4 voxels goes to `sink(frame index, lz, ly, lx0, values)`.  Frame
 // lists that step by 0 or 1 stream each control's keys; other non-decreasing lists (`monotone`)
 // walk a cursor; anything else, or keys that do not strictly increase, uses the reference's search.
 template <class M, class Sink, int NW = kLeafWarps>
@@ -153,19 +152,24 @@ __device__ __forceinline__ void leaf_decode(const DeviceAsset& a, const M& m, co
     const int Ctot = Cc + Cf;
     // frames per batch: as many as the control buffer holds, rounded down to a multiple of the
     // warp count when that still leaves a full round (each warp reconstructs whole frames)
-    int nb_max = min(nframes, kLeafCtrlBudget / max(Ctot, 1));
+    const int Cs = (Ctot + 3) & ~3;   // a frame's controls, 16-byte aligned
+    int nb_max = min(nframes, kLeafCtrlBudget / max(Cs, 1));
     if (nb_max < nframes && nb_max > NW) nb_max -= nb_max % NW;
     const bool stream = steps01 && (e.info & kFlagSorted) != 0u;
     const bool cursor = !stream && monotone && (e.info & kFlagSorted) != 0u;
     const bool plain = !occ && G.w == 8 && G.h == 8 && G.d == 8;
     const int ly = (lane >> 1) & 7, lx0 = 4 * (lane & 1);
+    // GRID4 and Mode2 leaves with 4^3 controls take the specialised path's trilinear, whose lanes hold
+    // layers i and 7 - i
+    const bool grid4 = cres == 4 && !fine;
+    auto layer = [&](int i) { return grid4 ? (lane >= 16 ? 7 - i : i) : 2 * i + (lane >> 4); };
     uint64_t mask[4] = {0, 0, 0, 0};
     uint32_t pref[4] = {0, 0, 0, 0};
     if (occ) {
         const uint64_t ob = base + 8u + e.coarse_bytes;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const uint32_t g = (uint32_t)(2 * i + (lane >> 4));
+            const uint32_t g = (uint32_t)layer(i);
             mask[i] = ((uint64_t)m((uint32_t)((ob + 8u * g + 4u) >> 2)) << 32) | m((uint32_t)((ob + 8u * g) >> 2));
             pref[i] = (m((uint32_t)((ob + 64u + 2u * g) >> 2)) >> ((g & 1u) * 16u)) & 0xFFFFu;
         }
@@ -181,14 +185,14 @@ __device__ __forceinline__ void leaf_decode(const DeviceAsset& a, const M& m, co
         auto run_unit = [&](int c, int j0, int j1) {
             const StreamRef st = c < Cc ? cs : (fine ? fs : ss);
             const uint32_t ci = (uint32_t)(c < Cc ? c : c - Cc);
-            float* dst = s.ctrl + j0 * Ctot + c;
+            float* dst = s.ctrl + j0 * Cs + c;
             if (stream) {
                 const uint32_t bin0 = st.bins == 8u ? s.b8[fb0 + j0] : s.b4[fb0 + j0];
-                m_control_stream(m, st, ci, s.fr + fb0 + j0, bin0, j1 - j0, dst, Ctot, s.rcp);
+                m_control_stream(m, st, ci, s.fr + fb0 + j0, bin0, j1 - j0, dst, Cs, s.rcp);
             } else {
                 const FrameBatch fb{s.fr + fb0 + j0, s.b8 + fb0 + j0, s.b4 + fb0 + j0, j1 - j0};
-                if (cursor) m_control_cursor(m, st, ci, fb, dst, Ctot);
-                else m_control_search(m, st, ci, fb, dst, Ctot);
+                if (cursor) m_control_cursor(m, st, ci, fb, dst, Cs);
+                else m_control_search(m, st, ci, fb, dst, Cs);
             }
         };
         const int c0 = Ctot > NT ? NT : 0;   // controls [0, c0) are owned whole
@@ -204,9 +208,17 @@ __device__ __forceinline__ void leaf_decode(const DeviceAsset& a, const M& m, co
         __syncthreads();
         // 2. voxels
         for (int j = warp; j < nb; j += NW) {
-            const float* g = s.ctrl + j * Ctot;
+            const float* g = s.ctrl + j * Cs;
             float4 q[4];
-            if (cres >= 2) trilinear_quads_ptr(s.w[0], x2, y4, g, cres, lane, q);
+            if (grid4) {
+                float4 y[kGridRows<4>];
+                grid_x<4>(s.lanes[0], g, reinterpret_cast<float*>(x2), lane);
+                __syncwarp();
+                grid_y<4>(s.lanes[0], reinterpret_cast<const float*>(x2), lane, y);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) q[i] = grid_z<4>(s.lanes[0], y, lane, i);
+                __syncwarp();   // the x rows are read before the next frame overwrites them
+            } else if (cres >= 2) trilinear_quads_ptr(s.w[0], x2, y4, g, cres, lane, q);
             else constant_quads(g, cres, q);
             if (fine) {
                 float4 qf[4];
@@ -222,12 +234,12 @@ __device__ __forceinline__ void leaf_decode(const DeviceAsset& a, const M& m, co
             const int fi = fb0 + j;
             if (plain) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) sink(fi, lane, i, q[i]);
+                for (int i = 0; i < 4; ++i) sink(fi, layer(i), ly, lx0, q[i]);
                 continue;
             }
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const int lz = 2 * i + (lane >> 4);
+                const int lz = layer(i);
                 float v[4] = {q[i].x, q[i].y, q[i].z, q[i].w};
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
@@ -240,7 +252,7 @@ __device__ __forceinline__ void leaf_decode(const DeviceAsset& a, const M& m, co
                     if (occ && !in_occ && v[k] < 0.0f) v[k] = 0.0f;
                     if (lx0 + k >= G.w || ly >= G.h || lz >= G.d) v[k] = 0.0f;
                 }
-                sink(fi, lane, i, make_float4(v[0], v[1], v[2], v[3]));
+                sink(fi, lz, ly, lx0, make_float4(v[0], v[1], v[2], v[3]));
             }
         }
         __syncthreads();
@@ -338,7 +350,7 @@ __device__ __noinline__ void leaf_decode_general(const DeviceAsset& a, M m, Leaf
 // stage, or (GLOBAL_KEYS: a leaf larger than the stage) straight from the payload through L1 --
 // the same byte offsets from the 16-byte-aligned window start a0; the payload's 16-byte tail
 // padding keeps the second word of the last key read inside the allocation.
-template <bool FINE, bool DENSE, bool GLOBAL_KEYS>
+template <int KIND, bool DENSE, bool GLOBAL_KEYS>
 __device__ __noinline__ void leaf_decode_fast_call(const DeviceAsset& a, LeafEntry e, uint32_t lb, uint64_t a0,
                                                    int nframes, LeafGeom G, float* __restrict__ out,
                                                    uint64_t frame_stride)
@@ -347,12 +359,15 @@ __device__ __noinline__ void leaf_decode_fast_call(const DeviceAsset& a, LeafEnt
     const LeafSmem s = leaf_layout<kDecWarps>(dyn);
     const QuadSink<DENSE> sink{out, frame_stride, G.li, a.g.width, a.g.height, G.bx, G.by, G.bz, G.w, G.h, G.d};
     const uint8_t* st = GLOBAL_KEYS ? reinterpret_cast<const uint8_t*>(a.payload) + a0 : s.stage;
-    leaf_decode_fast<FINE, kDecWarps>(st, lb, s, e, nframes, G, sink);
+    if constexpr (KIND == kFastShell) leaf_decode_shell<kDecWarps>(st, lb, s, e, nframes, G, sink);
+    else leaf_decode_fast<KIND == kFastFine6, kDecWarps>(st, lb, s, e, nframes, G, sink);
 }
 
-// GRID4 / FINE6 leaves of the common shape take leaf_decode_fast (rt_leaf_fast.cuh), staged or
+// GRID4, FINE6 and Mode2 leaves of the common shapes take rt_leaf_fast.cuh's paths, staged or
 // (GLOBAL_FALLBACK) from global memory; every other leaf the general leaf_decode.
-template <bool DENSE, bool GLOBAL_FALLBACK>
+// SHELL: with the Mode2 path, for assets with such leaves; its call in the kernel costs the other two
+// paths registers (fire, 32 frames: 313 us with it, 269 without).
+template <bool DENSE, bool GLOBAL_FALLBACK, bool SHELL>
 __global__ void __launch_bounds__(kDecThreads, 2) decode_leaf_kernel(const __grid_constant__ DeviceAsset a,
                                                                      FrameList fl, float* __restrict__ out,
                                                                      uint64_t frame_stride, unsigned long long* work,
@@ -439,7 +454,7 @@ __global__ void __launch_bounds__(kDecThreads, 2) decode_leaf_kernel(const __gri
         if (skip) {
             if (st != kOk && tid == 0) record_error(a.err, leaf, st);
             for (int idx = tid; idx < fl.n * 128; idx += kDecThreads)
-                store_quad<DENSE>(a, G, out, frame_stride, idx >> 7, (idx & 127) & 31, (idx & 127) >> 5,
+                store_quad<DENSE>(a, G, out, frame_stride, idx >> 7, (idx & 127) >> 4, (idx >> 1) & 7, 4 * (idx & 1),
                                   make_float4(0.f, 0.f, 0.f, 0.f));
         } else if (!GLOBAL_FALLBACK && !staged) {   // the launcher never lets this happen
             if (tid == 0) record_error(a.err, leaf, kErrDecodeOob);
@@ -458,15 +473,19 @@ __global__ void __launch_bounds__(kDecThreads, 2) decode_leaf_kernel(const __gri
                 return;
             }
             if (staged) phase ^= 1u;
-            bool fine = false;
-            if (fast_leaf_shape(e, steps01, fine) && (staged || GLOBAL_FALLBACK)) {
+            const int kind = fast_leaf_shape(e, steps01);
+            if (kind != kFastNone && (SHELL || kind != kFastShell) && (staged || GLOBAL_FALLBACK)) {
                 const uint32_t lb = (uint32_t)(b0 - a0);
                 if (staged) {
-                    if (fine) leaf_decode_fast_call<true, DENSE, false>(a, e, lb, a0, fl.n, G, out, frame_stride);
-                    else leaf_decode_fast_call<false, DENSE, false>(a, e, lb, a0, fl.n, G, out, frame_stride);
+                    if constexpr (SHELL)
+                        if (kind == kFastShell) leaf_decode_fast_call<kFastShell, DENSE, false>(a, e, lb, a0, fl.n, G, out, frame_stride);
+                    if (kind == kFastFine6) leaf_decode_fast_call<kFastFine6, DENSE, false>(a, e, lb, a0, fl.n, G, out, frame_stride);
+                    else if (kind == kFastGrid4) leaf_decode_fast_call<kFastGrid4, DENSE, false>(a, e, lb, a0, fl.n, G, out, frame_stride);
                 } else if constexpr (GLOBAL_FALLBACK) {
-                    if (fine) leaf_decode_fast_call<true, DENSE, true>(a, e, lb, a0, fl.n, G, out, frame_stride);
-                    else leaf_decode_fast_call<false, DENSE, true>(a, e, lb, a0, fl.n, G, out, frame_stride);
+                    if constexpr (SHELL)
+                        if (kind == kFastShell) leaf_decode_fast_call<kFastShell, DENSE, true>(a, e, lb, a0, fl.n, G, out, frame_stride);
+                    if (kind == kFastFine6) leaf_decode_fast_call<kFastFine6, DENSE, true>(a, e, lb, a0, fl.n, G, out, frame_stride);
+                    else if (kind == kFastGrid4) leaf_decode_fast_call<kFastGrid4, DENSE, true>(a, e, lb, a0, fl.n, G, out, frame_stride);
                 }
             } else if (staged) {
                 const SharedWords m{reinterpret_cast<const uint32_t*>(s.stage), (uint32_t)(a0 >> 2)};
@@ -481,30 +500,38 @@ __global__ void __launch_bounds__(kDecThreads, 2) decode_leaf_kernel(const __gri
     }
 }
 
-template <bool DENSE, bool GF>
+template <bool DENSE, bool GF, bool SHELL>
 static int leaf_grid(uint32_t smem_bytes)
 {
     int dev = 0, sms = 0, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, decode_leaf_kernel<DENSE, GF>, kDecThreads, smem_bytes);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, decode_leaf_kernel<DENSE, GF, SHELL>, kDecThreads, smem_bytes);
     return sms * (per > 0 ? per : 1);
 }
 
-template <bool DENSE, bool GF>
+template <bool DENSE, bool GF, bool SHELL>
 static void launch_leaf_variant(const DeviceAsset& a, uint32_t seq, const FrameList& fl, float* out, uint64_t stride,
                                 int grid, cudaStream_t s)
 {
     const uint32_t smem = kDecFixed + a.g.stage_bytes + kStagePad;
-    cudaFuncSetAttribute(decode_leaf_kernel<DENSE, GF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const int g = grid > 0 ? grid : leaf_grid<DENSE, GF>(smem);
+    cudaFuncSetAttribute(decode_leaf_kernel<DENSE, GF, SHELL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const int g = grid > 0 ? grid : leaf_grid<DENSE, GF, SHELL>(smem);
     unsigned long long* slot = a.work + seq % kWorkSlots;
     // Inside a stream capture the epoch is frozen into the graph: every replay starts from a
     // cleared slot instead (a graph is never replayed concurrently with itself).
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusActive)
         cudaMemsetAsync(slot, 0, sizeof(unsigned long long), s);
-    decode_leaf_kernel<DENSE, GF><<<g, kDecThreads, smem, s>>>(a, fl, out, stride, slot, seq + 1u);
+    decode_leaf_kernel<DENSE, GF, SHELL><<<g, kDecThreads, smem, s>>>(a, fl, out, stride, slot, seq + 1u);
+}
+
+template <bool DENSE, bool GF>
+static void launch_leaf_shell(const DeviceAsset& a, uint32_t seq, const FrameList& fl, float* out, uint64_t stride,
+                              int grid, cudaStream_t s)
+{
+    if (a.g.mode2) launch_leaf_variant<DENSE, GF, true>(a, seq, fl, out, stride, grid, s);
+    else launch_leaf_variant<DENSE, GF, false>(a, seq, fl, out, stride, grid, s);
 }
 
 static void launch_rt_leaf(const DeviceAsset& a, uint32_t seq, const FrameList& fl, float* out, uint64_t stride,
@@ -512,11 +539,11 @@ static void launch_rt_leaf(const DeviceAsset& a, uint32_t seq, const FrameList& 
 {
     const bool gf = a.g.max_window > a.g.stage_bytes;
     if (dense) {
-        if (gf) launch_leaf_variant<true, true>(a, seq, fl, out, stride, grid, s);
-        else launch_leaf_variant<true, false>(a, seq, fl, out, stride, grid, s);
+        if (gf) launch_leaf_shell<true, true>(a, seq, fl, out, stride, grid, s);
+        else launch_leaf_shell<true, false>(a, seq, fl, out, stride, grid, s);
     } else {
-        if (gf) launch_leaf_variant<false, true>(a, seq, fl, out, stride, grid, s);
-        else launch_leaf_variant<false, false>(a, seq, fl, out, stride, grid, s);
+        if (gf) launch_leaf_shell<false, true>(a, seq, fl, out, stride, grid, s);
+        else launch_leaf_shell<false, false>(a, seq, fl, out, stride, grid, s);
     }
 }
 

@@ -1,6 +1,7 @@
-// rt_leaf_fast.cuh -- the render decode kernel's specialised path for the two leaf shapes that make
-// up nearly every render-temporal asset: GRID4 (a 4^3 coarse grid) and FINE6 (4^3 coarse + 6^3
-// fine), FP16 key frames that strictly increase, over a timeline (frames stepping by 0 or 1).
+// rt_leaf_fast.cuh -- the render decode kernel's specialised paths for the leaf shapes that make up
+// nearly every render-temporal asset: GRID4 (a 4^3 coarse grid), FINE6 (4^3 coarse + 6^3 fine) and
+// Mode2 (4^3 coarse + shell), FP16 key frames that strictly increase, over a timeline (frames stepping
+// by 0 or 1).
 // Included by rt_kernel_leaf.cuh; the general leaf_decode there covers every other leaf.
 //
 // Same arithmetic as the general path, operation for operation (so the same bits):
@@ -50,9 +51,9 @@ __device__ __forceinline__ void fast_interval(KeyCursor& cu, const float* __rest
     cu.d = __fsub_rn(cu.vn, cu.vp);
 }
 
-// Set the cursor of control ci of the 8-bin stream at stage offset sbase (C controls, kf keys in
-// its pool) for first frame t0 in time bin bin0: the start of m_control_stream.
-__device__ __forceinline__ void fast_cursor_init(const uint8_t* __restrict__ st, uint32_t sbase, uint32_t C,
+// Set the cursor of control ci of the stream at stage offset sbase (C controls, `bins` = 8 or 4 time
+// bins, kf keys in its pool) for first frame t0 in time bin bin0: the start of m_control_stream.
+__device__ __forceinline__ void fast_cursor_init(const uint8_t* __restrict__ st, uint32_t sbase, uint32_t C, uint32_t bins,
                                                  uint32_t ci, uint32_t kf, int t0, uint32_t bin0,
                                                  const float* __restrict__ rcp, KeyCursor& cu)
 {
@@ -67,8 +68,8 @@ __device__ __forceinline__ void fast_cursor_init(const uint8_t* __restrict__ st,
     const uint32_t kc = (desc >> 16) & 0xFFu, ks = desc & 0xFFFFu;
     if (kc == 0u || ks + kc > kf) return;   // decodes to 0 (see decode_control, rt_search.cuh)
     cu.kc = (int)kc;
-    cu.kb = sbase + 12u * C + 3u * ks;      // descriptors (4 C) + 8-bin rows (8 C, 4-aligned)
-    const uint32_t hb = st[sbase + 4u * C + 8u * ci + bin0];
+    cu.kb = sbase + (4u + bins) * C + 3u * ks;   // descriptors (4 C) + bin rows (bins C, 4-aligned)
+    const uint32_t hb = st[sbase + 4u * C + bins * ci + bin0];
     uint32_t k = hb < kc - 1u ? hb : kc - 1u;
     if ((int)st[cu.kb + 3u * k] > t0) {
         uint32_t lo = 0, hi = k;
@@ -269,20 +270,22 @@ __device__ __forceinline__ float4 grid_z(const LaneWeights& w, const float4 (&y)
     return lerp4(y[n], y[n + 1], f, s);
 }
 
-// Can leaf_decode_fast take this leaf?  (Staged, timeline frames, strictly increasing FP16 keys
-// without NaN, coarse resolution 4, no Mode2 shell, and fine resolution 6 when there is a fine
-// stream.)
-__device__ __forceinline__ bool fast_leaf_shape(const LeafEntry& e, bool steps01, bool& fine)
+// The specialised path of a leaf, if it has one.  (Staged, timeline frames, strictly increasing FP16 keys
+// without NaN, coarse resolution 4, and alone, with a fine stream of resolution 6, or with a Mode2
+// occupancy and its shell.)
+enum : int { kFastNone, kFastGrid4, kFastFine6, kFastShell };
+__device__ __forceinline__ int fast_leaf_shape(const LeafEntry& e, bool steps01)
 {
     const uint32_t need = kFlagSorted | kFlagHalfPlain;
-    if (!steps01 || (e.info & need) != need || (e.info & (kFlagOccClamp | kFlagShell)) != 0u) return false;
-    if (((e.header >> 6) & 7u) != 4u || ((e.header >> 2) & 3u) == 1u) return false;
-    fine = (e.info & kFlagFine) != 0u;
-    return !fine || (((e.header >> 9) & 7u) == 6u && ((e.header >> 4) & 3u) != 1u);
+    if (!steps01 || (e.info & need) != need || ((e.header >> 6) & 7u) != 4u || ((e.header >> 2) & 3u) == 1u) return kFastNone;
+    const bool fcodec_ok = ((e.header >> 4) & 3u) != 1u;
+    if (e.info & kFlagOccClamp) return (e.info & kFlagFine) == 0u && ((e.info & kFlagShell) == 0u || fcodec_ok) ? kFastShell : kFastNone;
+    if ((e.info & kFlagFine) == 0u) return (e.info & kFlagShell) == 0u ? kFastGrid4 : kFastNone;
+    return ((e.header >> 9) & 7u) == 6u && fcodec_ok ? kFastFine6 : kFastNone;
 }
 
 // Decode one staged leaf of the fast shape for all nframes frames of the launch (NW warps; the
-// leaf's bytes start at stage offset lb).  Quads go to sink(frame index, lane, quad, values).
+// leaf's bytes start at stage offset lb).  Quads go to sink(frame index, lz, ly, lx0, values).
 // Per lane and slot the voxel phase holds one quad at a time.
 template <bool FINE, int NW, class Sink>
 __device__ __forceinline__ void leaf_decode_fast(const uint8_t* __restrict__ st, uint32_t lb, const LeafSmem& s,
@@ -309,7 +312,7 @@ __device__ __forceinline__ void leaf_decode_fast(const uint8_t* __restrict__ st,
     if (unit && f_lo < f_hi) {
         const uint32_t sbase = lb + 8u + (is_fine ? e.coarse_bytes : 0u);
         const uint32_t kf = is_fine ? (e.kf >> 16) : (e.kf & 0xFFFFu);
-        fast_cursor_init(st, sbase, C, ci, kf, s.fr[f_lo], s.b8[f_lo], s.rcp, cu);
+        fast_cursor_init(st, sbase, C, 8u, ci, kf, s.fr[f_lo], s.b8[f_lo], s.rcp, cu);
     }
     const bool plain = G.w == 8 && G.h == 8 && G.d == 8;
     float* xc = reinterpret_cast<float*>(s.x2 + warp * 196);   // x rows: 128 floats, and 288 in the y rows' place
@@ -357,6 +360,82 @@ __device__ __forceinline__ void leaf_decode_fast(const uint8_t* __restrict__ st,
                 sink(fi, lz, ly, lx0, v);
             }
             __syncwarp();   // the tables are read before the next slot overwrites them
+        }
+        __syncthreads();
+    }
+}
+
+// The same for a Mode2 leaf: 64 coarse and up to 512 shell controls, one or two cursors per thread, carried
+// across the batches as above (the general path started every control's cursor anew for each batch of
+// some eight frames; 32 frames of a 128^3 level set 246 -> 186 us).  A lane's four quads of occupancy do not change from frame to frame: the four
+// bits of a quad and the index of its first shell control are one register.
+template <int NW, class Sink>
+__device__ __forceinline__ void leaf_decode_shell(const uint8_t* __restrict__ st, uint32_t lb, const LeafSmem& s,
+                                                  const LeafEntry& e, int nframes, const LeafGeom& G, const Sink& sink)
+{
+    static_assert(64 + 512 <= 2 * 32 * NW, "two controls per thread");
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool shell = (e.info & kFlagShell) != 0u;
+    const uint32_t C2 = shell ? entry_shell_active(e) : 0u;
+    const int CT = 64 + (int)C2, Cs = (CT + 3) & ~3;
+    int m = min(kLeafCtrlBudget / Cs, nframes);   // frames per batch
+    if (m > NW) m -= m % NW;                      // whole voxel rounds
+    const int c1 = tid + 32 * NW;
+    const bool on0 = tid < CT, on1 = c1 < CT;
+    KeyCursor u0, u1;
+    auto init = [&](int c, KeyCursor& cu) {
+        const bool first = c < 64;
+        fast_cursor_init(st, lb + (first ? 8u : e.shell_off), first ? 64u : C2, first ? 8u : 4u,
+                         (uint32_t)(first ? c : c - 64), first ? e.kf & 0xFFFFu : e.kf >> 16, s.fr[0],
+                         first ? s.b8[0] : s.b4[0], s.rcp, cu);
+    };
+    if (on0) init(tid, u0);
+    if (on1) init(c1, u1);
+    const bool plain = G.w == 8 && G.h == 8 && G.d == 8;
+    const int ly = (lane >> 1) & 7, lx0 = 4 * (lane & 1);
+    uint32_t occ[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {   // mask[lz], then prefix[lz], of the occupancy after the coarse stream
+        const int lz = lane >= 16 ? 7 - i : i;
+        const uint8_t* ob = st + lb + 8u + e.coarse_bytes;
+        const uint32_t* mw = reinterpret_cast<const uint32_t*>(ob + 8 * lz);
+        const uint64_t mask = ((uint64_t)mw[1] << 32) | mw[0];
+        const uint32_t pref = (*reinterpret_cast<const uint32_t*>(ob + 64 + 4 * (lz >> 1)) >> ((lz & 1) * 16)) & 0xFFFFu;
+        const uint32_t bit = (uint32_t)(8 * ly + lx0);
+        occ[i] = ((uint32_t)(mask >> bit) & 15u) << 16 | (64u + pref + (uint32_t)__popcll(mask & ((1ull << bit) - 1ull)));
+    }
+    float* xc = reinterpret_cast<float*>(s.x2 + warp * 196);
+    for (int b0 = 0; b0 < nframes; b0 += m) {
+        const int mb = min(m, nframes - b0);
+        if (on0)
+            for (int j = 0; j < mb; ++j) s.ctrl[j * Cs + tid] = fast_cursor_step(u0, st, s.fr[b0 + j], s.rcp);
+        if (on1)
+            for (int j = 0; j < mb; ++j) s.ctrl[j * Cs + c1] = fast_cursor_step(u1, st, s.fr[b0 + j], s.rcp);
+        __syncthreads();
+        for (int j = warp; j < mb; j += NW) {
+            const float* g = s.ctrl + j * Cs;
+            grid_x<4>(s.lanes[0], g, xc, lane);
+            __syncwarp();
+            float4 y[kGridRows<4>];
+            grid_y<4>(s.lanes[0], xc, lane, y);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float4 z = grid_z<4>(s.lanes[0], y, lane, i);
+                float q[4] = {z.x, z.y, z.z, z.w};
+                const float* v = g + (occ[i] & 0xFFFFu);
+                const int lz = lane >= 16 ? 7 - i : i;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if ((occ[i] >> (16 + k)) & 1u) {
+                        if (shell) q[k] = __fadd_rn(q[k], *v++);
+                    } else if (q[k] < 0.0f) {
+                        q[k] = 0.0f;
+                    }
+                    if (!plain && (ly >= G.h || lz >= G.d || lx0 + k >= G.w)) q[k] = 0.0f;
+                }
+                sink(b0 + j, lz, ly, lx0, make_float4(q[0], q[1], q[2], q[3]));
+            }
+            __syncwarp();   // the x rows are read before the next frame overwrites them
         }
         __syncthreads();
     }
