@@ -539,8 +539,8 @@ WINDOW_ASSET = os.path.join(ROOT, "assets", "mix_sci.vbtp")
 
 def run_window(args, local_rank, reps=10):
     """(d) on the scientific field (config-5 scene, 128^3 x 64): the whole 64-frame timeline as
-    one tensor-core window per leaf (vbt_decode_window) against the exact per-frame decode of the
-    same frames (vbt_decode_cache, 64 frames per launch); device time per timeline, and the error
+    one window per leaf (vbt_decode_window) against the cache decode of the same frames
+    (vbt_decode_cache, 64 frames per launch); device time per timeline, and the error
     of both against the FP64 oracle, relative to the field range."""
     import torch
     import vbt_b200 as vbt
@@ -576,7 +576,7 @@ def run_window(args, local_rank, reps=10):
     vox = L * 512 * n
     a.close()
     return {"asset": os.path.basename(path), "frames": n, "leaves": L,
-            "tensor_core_window": {"ms_per_timeline": win_ms, "voxels_per_s": vox / (win_ms * 1e-3),
+            "window": {"ms_per_timeline": win_ms, "voxels_per_s": vox / (win_ms * 1e-3),
                                    "max_abs_err_rel_range": mx_w / rng, "rms_err_rel_range": rms_w / rng,
                                    "products": "split-BF16: exact S' x three BF16 terms of C, FP32 accumulate"},
             "fp32_per_frame": {"ms_per_timeline": ref_ms, "voxels_per_s": vox / (ref_ms * 1e-3),
@@ -590,9 +590,8 @@ RENDER_WINDOW_ASSETS = ["mix_fire_density", "mix_fire_flames", "mix_fire_tempera
 
 def run_window_render(args, local_rank, reps=5):
     """(d) on the fire (config-3 scene, three fields 128 x 128 x 192 x 40): 16-frame timeline
-    windows per active leaf (vbt_decode_window: exact voxels at the union of key-frame knots, hat
-    basis x knot coefficients on the tensor cores) over the whole timeline, against the exact
-    per-frame decode of the same frames (vbt_decode_cache, 16 frames per launch); device time and
+    windows per active leaf (vbt_decode_window) over the whole timeline, against the cache decode
+    of the same frames (vbt_decode_cache, 16 frames per launch); device time and
     the error of both against the FP64 oracle, relative to each field's range."""
     import torch
     import vbt_b200 as vbt
@@ -633,7 +632,7 @@ def run_window_render(args, local_rank, reps=5):
         rng = hi - lo
         vox = A * 512 * n
         out[name] = {"frames": n, "windows": len(starts), "active_leaves": A,
-                     "tensor_core_window": {"ms": win_ms, "voxels_per_s": vox / (win_ms * 1e-3),
+                     "window": {"ms": win_ms, "voxels_per_s": vox / (win_ms * 1e-3),
                                             "max_abs_err_rel_range": mx_w / rng, "rms_err_rel_range": rms_w / rng},
                      "fp32_per_frame": {"ms": ref_ms, "voxels_per_s": vox / (ref_ms * 1e-3),
                                         "max_abs_err_rel_range": mx_r / rng, "rms_err_rel_range": rms_r / rng},
@@ -1007,8 +1006,8 @@ def cache_timeline(torch, a, dev, W=16, reps=2):
 
 
 def window_vs_exact(torch, a, dev, W=16):
-    """(d) over the whole timeline in W-frame windows per active leaf: the tensor-core window
-    (vbt_decode_window) and the exact per-frame decode (vbt_decode_cache), device time of each,
+    """(d) over the whole timeline in W-frame windows per active leaf: the window
+    (vbt_decode_window) and the cache decode (vbt_decode_cache), device time of each,
     and the error of each against the FP64 oracle relative to the field's range."""
     T, A = a.frames, a.active_count
     starts = list(range(0, T - W + 1, W))
@@ -1034,7 +1033,7 @@ def window_vs_exact(torch, a, dev, W=16):
     vox = A * 512 * W * len(starts)
     del win, ref
     return {"windows": len(starts), "frames": W * len(starts), "oracle_range": [lo, hi],
-            "tensor_core_window": {"ms": win_ms, "voxels_per_s": vox / (win_ms * 1e-3),
+            "window": {"ms": win_ms, "voxels_per_s": vox / (win_ms * 1e-3),
                                    "max_abs_err_rel_range": stats["window"][0] / rng,
                                    "rms_err_rel_range": (stats["window"][1] / len(starts)) ** 0.5 / rng},
             "fp32_per_frame": {"ms": ref_ms, "voxels_per_s": vox / (ref_ms * 1e-3),

@@ -330,8 +330,8 @@ class Asset:
 
     def decode_window(self, t0, n, out, frame_stride=None, stream=None):
         """(d) window decode of frames [t0, t0 + n) into `out` in the cache layout: scientific assets
-        n <= 64, every leaf, by the exact frames kernel; render assets n <= 64 as 16-frame windows on
-        the tensor cores, the active leaves of the current page table (build it first)."""
+        n <= 64, every leaf; render assets n <= 64, the active leaves of the current page table
+        (build it first); the values of decode_cache."""
         stride = self.leaf_count * 512 if frame_stride is None else frame_stride
         _check(_lib.vbt_decode_window(self._h, t0, n, _addr(out), stride, _stream(stream)))
 

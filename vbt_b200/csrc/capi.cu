@@ -604,9 +604,11 @@ int vbt_decode_window(vbt_asset* a, int t0, int n, float* d_out, uint64_t frame_
     if ((reinterpret_cast<uintptr_t>(d_out) & 15u) != 0u || (frame_stride & 3u) != 0u)
         return fail(VBT_STATUS_INVALID_ARGUMENT, "output must be 16-byte aligned, frame_stride a multiple of 4");
     DeviceGuard guard(a->device);
-    launch_render_window(a->dev, a->launch_seq.fetch_add(1), t0, n, d_out, frame_stride,
-                         static_cast<cudaStream_t>(stream));
-    return check_launch("render_window_kernel");
+    int frames[64];
+    for (int i = 0; i < n; ++i) frames[i] = t0 + i;
+    launch_decode_cache(a->dev, a->launch_seq.fetch_add(1), frames, n, d_out, frame_stride, 0,
+                        static_cast<cudaStream_t>(stream));
+    return check_launch("cache decode");
 }
 
 int vbt_window_error(vbt_asset* a, int t0, int n, const float* d_values, uint64_t frame_stride, double* stats,

@@ -1268,8 +1268,6 @@ void launch_key_division_check(uint32_t b_max, unsigned long long* d_out, cudaSt
 
 }  // namespace vbtb
 
-// (d) window decode of scientific leaves on the tensor cores: sci_window.cuh
-#include <cuda_bf16.h>
-
+// (d) windows and their error oracles
 #include "sci_window.cuh"
 #include "render_window.cuh"

@@ -113,8 +113,6 @@ void launch_sci_window(const DeviceAsset& a, int t0, int n, float* out, uint64_t
 // (double), stats[2] / stats[3] oracle min / max (order-preserving bits).
 void launch_control_cache(const DeviceAsset& a, const int* frames, int nframes, float* out, uint64_t stride,
                           cudaStream_t s);
-void launch_render_window(const DeviceAsset& a, uint32_t seq, int t0, int n, float* out, uint64_t frame_stride,
-                          cudaStream_t s);
 void launch_render_window_oracle(const DeviceAsset& a, int t0, int n, const float* vals, uint64_t frame_stride,
                                  unsigned long long* stats, cudaStream_t s);
 void launch_key_division_check(uint32_t b_max, unsigned long long* d_out, cudaStream_t s);

@@ -12,8 +12,6 @@
 
 namespace vbtb {
 
-constexpr int kLeafThreads = 256;   // the render window kernel (render_window.cuh)
-constexpr int kLeafWarps = kLeafThreads / 32;
 constexpr int kDecWarps = 9;         // the decode kernel: 288 threads, one per FINE6 control
 constexpr int kDecThreads = 32 * kDecWarps;
 constexpr int kLeafCtrlBudget = 3072;   // floats: frames x controls of one batch
@@ -21,7 +19,6 @@ constexpr uint32_t leaf_fixed_bytes(int nw)
 {
     return 16 + 6 * kMaxLaunchFrames + 576 + nw * 196 * 8 + nw * 112 * 16 + kLeafCtrlBudget * 4 + 256 * 4 + 5120;
 }
-constexpr uint32_t kLeafFixed = leaf_fixed_bytes(kLeafWarps);
 constexpr uint32_t kDecFixed = leaf_fixed_bytes(kDecWarps);
 constexpr uint32_t kStagePad = 16;   // readable bytes past the largest staged window
 static_assert(kDecFixed == kLeafFixedBytes, "host stage sizing must match the kernel's shared-memory layout");
@@ -41,7 +38,7 @@ struct LeafSmem {
 };
 
 // Shared-memory layout for NW warps (x-lerp and y-lerp rows per warp).
-template <int NW = kLeafWarps>
+template <int NW>
 __device__ __forceinline__ LeafSmem leaf_layout(uint8_t* dyn)
 {
     LeafSmem s;
@@ -132,7 +129,7 @@ struct QuadSink {
 // warps; each finished quad of 4 voxels goes to `sink(frame index, lz, ly, lx0, values)`.  Frame
 // lists that step by 0 or 1 stream each control's keys; other non-decreasing lists (`monotone`)
 // walk a cursor; anything else, or keys that do not strictly increase, uses the reference's search.
-template <class M, class Sink, int NW = kLeafWarps>
+template <class M, class Sink, int NW>
 __device__ __forceinline__ void leaf_decode(const DeviceAsset& a, const M& m, const LeafSmem& s, const LeafEntry& e,
                                             int nframes, bool steps01, bool monotone, const LeafGeom& G,
                                             const Sink& sink)

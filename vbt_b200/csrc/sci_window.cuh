@@ -1,82 +1,14 @@
-// sci_window.cuh -- the FP64 error oracle of scientific windows, the window launcher, and the tcgen05
-// helpers of the render windows (render_window.cuh).  Included by kernels.cu (it uses that file's
-// scientific helpers).
+// sci_window.cuh -- the FP64 error oracle of scientific windows and the window launcher.  Included by
+// kernels.cu (it uses that file's scientific helpers).
 //
 // A scientific window is decoded by the exact frames kernel (sci_frames.cuh): with a leaf's
 // coefficients, weights and events in registers a frame costs less on the CUDA cores than splitting
 // its controls into three BF16 terms, 48 MMAs per leaf-window and an epilogue that adds corners and
 // events -- 64 frames of a 128^3 field on a B200: 162 us against 499 us for the contraction -- and the
 // values are the exact path's own.
-//
-// Shared-memory operand layout of the MMA helpers (canonical K-major, no swizzle): per K step, core
-// matrices of 8 rows x 16 bytes; the two 8-element K halves 128 bytes apart (leading byte offset),
-// 8-row groups 256 bytes apart (stride byte offset).
 #pragma once
 
 namespace vbtb {
-
-__device__ __forceinline__ uint32_t win_smem_u32(const void* p)
-{
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-// Shared-memory matrix descriptor: start >> 4 [0,14), LBO >> 4 [16,30), SBO >> 4 [32,46),
-// version 1 [46,48), no swizzle [61,64).
-__device__ __forceinline__ uint64_t win_desc(uint32_t saddr)
-{
-    return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)(128u >> 4) << 16) | ((uint64_t)(256u >> 4) << 32) |
-           (1ull << 46);
-}
-
-// Byte offset of (row, k) inside one K step of a K-major operand tile.
-__device__ __forceinline__ uint32_t win_off(uint32_t row, uint32_t k)
-{
-    return (row >> 3) * 256u + (k >> 3) * 128u + (row & 7u) * 16u + (k & 7u) * 2u;
-}
-
-__device__ __forceinline__ uint16_t win_bf16_bits(float x)
-{
-    const __nv_bfloat16 b = __float2bfloat16_rn(x);
-    return *reinterpret_cast<const uint16_t*>(&b);
-}
-__device__ __forceinline__ float win_bf16_val(uint16_t bits)
-{
-    return __uint_as_float((uint32_t)bits << 16);
-}
-
-__device__ __forceinline__ void win_tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void win_tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-// D[tmem] (+)= A[desc] x B[desc], kind::f16 (BF16 inputs, FP32 accumulate).
-__device__ __forceinline__ void win_mma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t acc)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc)
-        : "memory");
-}
-
-__device__ __forceinline__ void win_commit(uint64_t* bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(win_smem_u32(bar))
-                 : "memory");
-}
-
-// 16 consecutive FP32 columns of this thread's tensor-memory lane.
-__device__ __forceinline__ void win_ld16(uint32_t taddr, float (&v)[16])
-{
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
 
 // FP64 error oracle of a window (any scientific output of frames [t0, t0 + n) in the cache
 // layout; voxels outside a boundary leaf's extent must be 0): per voxel and frame the reference
