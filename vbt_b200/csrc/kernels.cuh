@@ -48,7 +48,7 @@ constexpr int kMaxLaunchFrames = 128;
 // barrier, frame tables, axis weights, 9 warps x (x-lerp + y-lerp rows), 3072-float controls,
 // reciprocal table, lane weights).
 constexpr uint32_t kLeafFixedBytes =
-    16 + 6 * kMaxLaunchFrames + 576 + 9 * 196 * 8 + 9 * 112 * 16 + 3072 * 4 + 256 * 4 + 5120;
+    16 + 6 * kMaxLaunchFrames + 576 + 9 * 196 * 8 + 9 * 112 * 16 + 3072 * 4 + 256 * 4 + 512;
 
 constexpr int kWalkThreads = 256;
 constexpr int kWalkTile = 256;   // leaves per walker CTA (one scan element per thread)

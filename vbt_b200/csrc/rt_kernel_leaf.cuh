@@ -17,7 +17,7 @@ constexpr int kDecThreads = 32 * kDecWarps;
 constexpr int kLeafCtrlBudget = 3072;   // floats: frames x controls of one batch
 constexpr uint32_t leaf_fixed_bytes(int nw)
 {
-    return 16 + 6 * kMaxLaunchFrames + 576 + nw * 196 * 8 + nw * 112 * 16 + kLeafCtrlBudget * 4 + 256 * 4 + 5120;
+    return 16 + 6 * kMaxLaunchFrames + 576 + nw * 196 * 8 + nw * 112 * 16 + kLeafCtrlBudget * 4 + 256 * 4 + 512;
 }
 constexpr uint32_t kDecFixed = leaf_fixed_bytes(kDecWarps);
 constexpr uint32_t kStagePad = 16;   // readable bytes past the largest staged window
@@ -52,7 +52,7 @@ __device__ __forceinline__ LeafSmem leaf_layout(uint8_t* dyn)
     s.ctrl = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(s.y4) + NW * 112 * 16);
     s.rcp = s.ctrl + kLeafCtrlBudget;
     s.lanes = reinterpret_cast<LaneWeights*>(s.rcp + 256);
-    s.stage = reinterpret_cast<uint8_t*>(s.rcp + 256) + 5120;
+    s.stage = reinterpret_cast<uint8_t*>(s.rcp + 256) + 512;
     return s;
 }
 

@@ -179,31 +179,29 @@ __device__ __forceinline__ float4 trilinear_z(const float4* __restrict__ w16, co
     return make_float4(lo2.x, lo2.y, hi2.x, hi2.y);
 }
 
-// A lane's weights of the grids with 4 and 6 controls, as rows of 32 lanes: x quad first / second, z rows
-// first / second, {y t, y 1 - t, y control}.  First and second in mirrored order for the upper halves
-// (lane & 1 for x, lane >> 4 for z).
+// The weights of a grid's lanes: x quad first / second by the half lane & 1, z rows first / second by the half
+// lane >> 4 (both in mirrored order for the upper half), {y t, y 1 - t, y control} by (lane >> 1) & 7.  Rows
+// per half instead of per lane leave 4.5 KB more of the shared memory to the leaf stage: a 256^3 plume whose
+// largest leaves lie there 512 -> 460 us (96 frames), one staged either way 466 -> 457.
 struct LaneWeights {
-    float4 xf[32], xs[32], zf[32], zs[32], y[32];
+    float4 xf[2], xs[2], zf[2], zs[2], y[8];
 };
+static_assert(2 * sizeof(LaneWeights) == 512, "their place in the leaf kernel's layout");
 
 __device__ __forceinline__ void fill_lane_weights(LaneWeights* w)   // a barrier follows
 {
-    for (int i = (int)threadIdx.x; i < 64; i += (int)blockDim.x) {
-        const int g = i >> 5, lane = i & 31, res = g == 0 ? 4 : 6;
-        float f[2][4], s[2][4];
-        for (int k = 0; k < 4; ++k)
-            for (int a = 0; a < 2; ++a) {
-                const bool up = a == 0 ? (lane & 1) != 0 : lane >= 16;
-                const AxisWeight aw = g_axis[axis_index(res, 8, up ? 7 - k : k)];
-                f[a][k] = up ? aw.t : aw.omt;
-                s[a][k] = up ? aw.omt : aw.t;
-            }
-        const AxisWeight ay = g_axis[axis_index(res, 8, (lane >> 1) & 7)];
-        w[g].xf[lane] = make_float4(f[0][0], f[0][1], f[0][2], f[0][3]);
-        w[g].xs[lane] = make_float4(s[0][0], s[0][1], s[0][2], s[0][3]);
-        w[g].zf[lane] = make_float4(f[1][0], f[1][1], f[1][2], f[1][3]);
-        w[g].zs[lane] = make_float4(s[1][0], s[1][1], s[1][2], s[1][3]);
-        w[g].y[lane] = make_float4(ay.t, ay.omt, __int_as_float((int)ay.i0), 0.0f);
+    const int i = (int)threadIdx.x;
+    if (i < 32) {   // grid, axis (x, z), half, position
+        const int g = i >> 4, up = (i >> 2) & 1, k = i & 3;
+        const AxisWeight aw = g_axis[axis_index(g == 0 ? 4 : 6, 8, up ? 7 - k : k)];
+        float4* f = (i >> 3) & 1 ? w[g].zf : w[g].xf;
+        float4* s = (i >> 3) & 1 ? w[g].zs : w[g].xs;
+        reinterpret_cast<float*>(f + up)[k] = up ? aw.t : aw.omt;
+        reinterpret_cast<float*>(s + up)[k] = up ? aw.omt : aw.t;
+    } else if (i < 48) {
+        const int g = (i >> 3) & 1, p = i & 7;
+        const AxisWeight ay = g_axis[axis_index(g == 0 ? 4 : 6, 8, p)];
+        w[g].y[p] = make_float4(ay.t, ay.omt, __int_as_float((int)ay.i0), 0.0f);
     }
 }
 
@@ -218,7 +216,7 @@ template <int R>
 __device__ __forceinline__ void grid_x(const LaneWeights& w, const float* __restrict__ g, float* __restrict__ x, int lane)
 {
     const bool up = (lane & 1) != 0;
-    const float4 f = w.xf[lane], s = w.xs[lane];
+    const float4 f = w.xf[lane & 1], s = w.xs[lane & 1];
 #pragma unroll
     for (int m = 0; m < (R == 4 ? 1 : 3); ++m) {
         const int row = (lane >> 1) + 16 * m;
@@ -252,7 +250,7 @@ constexpr int kGridRows = R == 4 ? 3 : 4;
 template <int R>
 __device__ __forceinline__ void grid_y(const LaneWeights& w, const float* __restrict__ x, int lane, float4 (&y)[kGridRows<R>])
 {
-    const float4 wy = w.y[lane];
+    const float4 wy = w.y[(lane >> 1) & 7];
     const float* r0 = x + 8 * __float_as_int(wy.z) + 4 * (lane & 1);
 #pragma unroll
     for (int n = 0; n < kGridRows<R>; ++n) {
@@ -265,7 +263,7 @@ __device__ __forceinline__ void grid_y(const LaneWeights& w, const float* __rest
 template <int R>
 __device__ __forceinline__ float4 grid_z(const LaneWeights& w, const float4 (&y)[kGridRows<R>], int lane, int i)
 {
-    const float f = reinterpret_cast<const float*>(&w.zf[lane])[i], s = reinterpret_cast<const float*>(&w.zs[lane])[i];
+    const float f = reinterpret_cast<const float*>(&w.zf[lane >> 4])[i], s = reinterpret_cast<const float*>(&w.zs[lane >> 4])[i];
     const int n = R == 4 ? (i == 3 ? 1 : 0) : (i == 3 ? 2 : i == 2 ? 1 : 0);
     return lerp4(y[n], y[n + 1], f, s);
 }
