@@ -590,6 +590,7 @@ __global__ void __launch_bounds__(R * R * R) control_fit_kernel(const float* __r
         }
         sv[t * NV + c] = v;
     }
+    if (RESID) __syncthreads();   // every thread has read the last staged frames: the spans take their place
     const Column<NV> col{sv + c, sm + c};
     float* grid = o.grid ? o.grid + ((unsigned long long)li * NV + (unsigned)c) * (unsigned)n : nullptr;
     const SeriesOut r = keyframe_series<NV>(col, stop + c, n, words, p, grid, 1ull);
