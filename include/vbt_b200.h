@@ -339,11 +339,13 @@ int vbt_build_page_table_noalloc(const uint32_t* d_offsets, const uint32_t* d_pa
 /* ---- (d) Window decode --------------------------------------------------------------------------
  * No counterpart in the reference.  Scientific assets (profile 2): the current-frame cache of
  * frames [t0, t0 + n), n <= 64, d_out[f * frame_stride + leaf * 512 + voxel] as vbt_decode_cache gives
- * it, every leaf and every generic leaf mode, by the same kernel.
+ * it, every leaf and every generic leaf mode, by the same kernel.  d_out may start at any float and
+ * frame_stride be any number from leaf_count * 512 on; with d_out 16-byte aligned and frame_stride a
+ * multiple of 4 the stores are 16 bytes wide.
  * Render-temporal assets (profile 1): frames [t0, t0 + n), n <= 64, d_out[f * frame_stride +
  * rank * 512 + voxel] over the active leaves of the current page table (vbt_build_page_table
- * first), the values of vbt_decode_cache by its kernels.  d_out 16-byte aligned, frame_stride a multiple
- * of 4.  vbt_window_error gives the values' error. */
+ * first), the values of vbt_decode_cache by its kernels.  Of these, d_out must be 16-byte aligned and
+ * frame_stride a multiple of 4.  vbt_window_error gives the values' error. */
 int vbt_decode_window(vbt_asset* asset, int t0, int n, float* d_out, uint64_t frame_stride, void* stream);
 /* FP64 error oracle on the GPU for any cache of frames [t0, t0 + n) (from vbt_decode_window or
  * vbt_decode_cache; render assets: the active ranks of the current page table): the reference

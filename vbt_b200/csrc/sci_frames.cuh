@@ -171,7 +171,9 @@ __device__ __forceinline__ bool sci_common_shape(const AssetGeom& g, const LeafE
 // events, temporal-basis residuals) go through the per-frame functions.
 // Four CTAs of 128 registers: with 96 registers and five, the spills and the wider spread of the writes
 // cost more than the warps hide (222 against 265 us).
-template <bool DENSE>
+// LOOSE: a cache that starts at any float, its frames any number of floats apart (an instantiation of its
+// own: the test in the one kernel costs an aligned window of 64 frames of 128^3 1.5 %).
+template <bool DENSE, bool LOOSE>
 __global__ void __launch_bounds__(kSciWarps * 32, 4) sci_frames_kernel(DeviceAsset a, FrameList fl, int chunk,
                                                                        float* __restrict__ out, uint64_t frame_stride)
 {
@@ -182,8 +184,10 @@ __global__ void __launch_bounds__(kSciWarps * 32, 4) sci_frames_kernel(DeviceAss
     const int ly = (lane >> 1) & 7, lx0 = 4 * (lane & 1);
     const bool hz = lane >= 16;
     const SciWeights<4> W(lane);
-    const bool aligned = !DENSE || ((a.g.width & 3u) == 0u && (frame_stride & 3u) == 0u &&
-                                    (reinterpret_cast<uintptr_t>(out) & 15u) == 0u);
+    // 16-byte stores: every quad of every frame on a 16-byte boundary
+    const bool aligned = DENSE ? (a.g.width & 3u) == 0u && (frame_stride & 3u) == 0u &&
+                                     (reinterpret_cast<uintptr_t>(out) & 15u) == 0u
+                               : !LOOSE;
     const int f0 = (int)blockIdx.y * chunk, n = min(chunk, fl.n - f0);
     for (uint64_t at = (uint64_t)blockIdx.x * kSciWarps + warp; at < n_leaves; at += (uint64_t)gridDim.x * kSciWarps) {
         const uint32_t rank = (uint32_t)at;
@@ -201,7 +205,7 @@ __global__ void __launch_bounds__(kSciWarps * 32, 4) sci_frames_kernel(DeviceAss
         const bool plain = whole && aligned;
         float* dst = fout + (hz ? 7u * plane : 0u) + (uint64_t)ly * row + (uint64_t)lx0;
         const int64_t zstep = hz ? -(int64_t)plane : (int64_t)plane;
-        // voxels lx .. lx + 3 of a row: in the cache whole quads, 0 outside the extent; in dense frames
+        // voxels lx .. lx + 3 of a row: in the cache all four, 0 outside the extent; in dense frames
         // what lies inside
         auto put = [&](int j, int y, int z, int lx, float4 v) {
             float* o = fout + (uint64_t)j * frame_stride + (uint64_t)z * plane + (uint64_t)y * row + (uint64_t)lx;
@@ -213,7 +217,14 @@ __global__ void __launch_bounds__(kSciWarps * 32, 4) sci_frames_kernel(DeviceAss
                     if (!in || lx + 2 >= w) v.z = 0.0f;
                     if (!in || lx + 3 >= w) v.w = 0.0f;
                 }
-                *reinterpret_cast<float4*>(o) = v;
+                if (aligned) {
+                    *reinterpret_cast<float4*>(o) = v;
+                } else {
+                    o[0] = v.x;
+                    o[1] = v.y;
+                    o[2] = v.z;
+                    o[3] = v.w;
+                }
             } else if (in) {
                 if (aligned && w == 8) {
                     *reinterpret_cast<float4*>(o) = v;
@@ -417,16 +428,19 @@ static void launch_sci_frames(const DeviceAsset& a, const FrameList& fl, float* 
         int dev = 0, sms = 0, per = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sci_frames_kernel<DENSE>, kSciWarps * 32, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sci_frames_kernel<DENSE, false>, kSciWarps * 32, 0);
         full = sms * (per > 0 ? per : 1);
     }
     const uint64_t warps = (uint64_t)full * kSciWarps, L = a.g.leaf_count;
     auto items = [&](int c) { return L * (uint64_t)((fl.n + c - 1) / c); };
     const int chunk = items(16) >= 12u * warps ? 16 : items(8) >= 2u * warps ? 8 : 4;
     const uint64_t most = (L + kSciWarps - 1) / kSciWarps;
-    sci_frames_kernel<DENSE><<<dim3((unsigned)(grid > 0 && (uint64_t)grid < most ? (uint64_t)grid : most),
-                                    (unsigned)((fl.n + chunk - 1) / chunk)),
-                               kSciWarps * 32, 0, s>>>(a, fl, chunk, out, stride);
+    const dim3 ctas((unsigned)(grid > 0 && (uint64_t)grid < most ? (uint64_t)grid : most),
+                    (unsigned)((fl.n + chunk - 1) / chunk));
+    if (!DENSE && ((stride & 3u) != 0u || (reinterpret_cast<uintptr_t>(out) & 15u) != 0u))
+        sci_frames_kernel<DENSE, !DENSE><<<ctas, kSciWarps * 32, 0, s>>>(a, fl, chunk, out, stride);
+    else
+        sci_frames_kernel<DENSE, false><<<ctas, kSciWarps * 32, 0, s>>>(a, fl, chunk, out, stride);
 }
 
 }  // namespace vbtb
