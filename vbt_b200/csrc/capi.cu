@@ -162,8 +162,11 @@ namespace vbtb {
 int set_last_error(int status, const std::string& msg) { return fail(status, msg); }
 }  // namespace vbtb
 
-// Launch-shape facts taken from a render-temporal image's route tags and leaf sizes (nothing is
-// read from the device):
+// Launch-shape facts taken from an image's leaf headers and sizes (nothing is read from the device).
+// Scientific:
+//  - wide: a leaf with more than four coefficients per control, a temporal-basis residual or codes of more than
+//    eight bits (the frames kernel that covers them).
+// Render-temporal:
 //  - sparse: fewer than half of the leaves non-EMPTY (the point-query kernel's shape hint);
 //  - mode2: a Mode2 leaf among them;
 //  - the shared-memory leaf stage of the render decode kernel: the largest 16-byte-aligned window
@@ -175,8 +178,18 @@ int set_last_error(int status, const std::string& msg) { return fail(status, msg
 static void image_shape(const vbt_header& h, const uint8_t* b, uint64_t off_off, uint64_t pay_off, uint64_t words,
                         AssetGeom& g, bool& sparse)
 {
-    if (h.profile_type == 2u) return;
     const uint8_t* off = b + off_off;
+    if (h.profile_type == 2u) {
+        g.wide = 0u;
+        for (uint32_t i = 0; i < h.leaf_count && g.wide == 0u; ++i) {
+            const uint64_t w0 = rd32(off + 4ull * i);
+            if (w0 >= words) continue;
+            const uint32_t hdr = rd32(b + pay_off + 4ull * w0);
+            const bool grid = (hdr & 3u) >= 2u;
+            g.wide = ((hdr >> 2) & 0x3Fu) > 3u || (grid && (((hdr >> 12) & 7u) == 1u || ((hdr >> 8) & 0xFu) > 8u)) ? 1u : 0u;
+        }
+        return;
+    }
     const uint32_t cap = ((233472u / 2u - 1024u - kLeafFixedBytes - 16u) / 1024u) * 1024u;
     uint64_t active = 0, maxw = 0, fits = 0, mode2 = 0;
     for (uint32_t i = 0; i < h.leaf_count; ++i) {
@@ -383,7 +396,9 @@ int vbt_asset_upload(vbt_asset* a, const void* file_bytes, uint64_t len, void* s
     bool sparse = a->sparse;
     image_shape(h, b, off_off, pay_off, a->dev.g.payload_words, g, sparse);
     DeviceGuard guard(a->device);
-    if (g.stage_bytes != a->dev.g.stage_bytes || g.max_window != a->dev.g.max_window) release_timeline_graphs(a);
+    if (g.stage_bytes != a->dev.g.stage_bytes || g.max_window != a->dev.g.max_window || g.mode2 != a->dev.g.mode2 ||
+        g.wide != a->dev.g.wide)
+        release_timeline_graphs(a);
     a->dev.g = g;
     a->sparse = sparse;
     cudaStream_t s = static_cast<cudaStream_t>(stream);

@@ -17,6 +17,7 @@ struct AssetGeom {
     uint32_t max_window;    // largest 16-byte-aligned window of a non-EMPTY leaf
     uint32_t sparse;        // 1: render-temporal with most leaves EMPTY (the point-query shape)
     uint32_t mode2;         // 1: some leaf is a Mode2 one (the streaming kernel with its path)
+    uint32_t wide;          // scientific, 1: leaves that need the WIDE frames kernel (sci_frames.cuh)
 };
 
 struct DeviceAsset {

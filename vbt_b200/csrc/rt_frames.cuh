@@ -42,11 +42,6 @@ __device__ __forceinline__ bool rt_common_shape(const LeafEntry& e)
     return (e.info & kFlagShell) == 0u || ((hdr >> 4) & 3u) != 1u;
 }
 
-__device__ __forceinline__ float4 add4(float4 a, float4 b)
-{
-    return make_float4(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z), __fadd_rn(a.w, b.w));
-}
-
 // Mode2: voxels bit0 .. bit0 + 3 of a layer with occupancy `mask` add their shell values (shell[0] =
 // the layer's first); the others are clamped at 0 from below.
 __device__ __forceinline__ float4 shell_quad(float4 v, uint64_t mask, uint32_t bit0, const float* shell)

@@ -23,12 +23,15 @@ namespace vbtb {
 
 constexpr int kSciChunk = 16;   // frames of one item at most
 constexpr int kSciWarps = 4;
+constexpr int kSciWideFrames = 4;   // frames whose controls a WIDE item forms together
+template <bool WIDE>
 struct __align__(16) SciWarpShared {
     union {
         struct {
-            float ctrl[64];          // control rows of 4
-            float x[16 * 8];         // x-lerped control rows
-            float residual[512];     // events of the frame (all 0 between frames), or the residual grid's rows of 4
+            float ctrl[WIDE ? kSciWideFrames * 64 : 64];   // control rows of 4 (WIDE: of four frames)
+            float x[16 * 8];                // x-lerped control rows
+            float residual[WIDE ? 1024 : 512];   // events of the frame (all 0 between frames), or residual grids of
+                                                 // 64, in rows of 4 (WIDE: the temporal-basis grids of the leaf)
         };
         float general[64 + 16 * 64];   // sci_decode_controls' values, for leaves of no common shape
     };
@@ -67,6 +70,14 @@ struct SciWeights {
 __device__ __forceinline__ float lerp_fs(float f, float s, float wf, float ws)
 {
     return __fadd_rn(__fmul_rn(f, wf), __fmul_rn(s, ws));
+}
+__device__ __forceinline__ float4 add4(float4 a, float4 b)
+{
+    return make_float4(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z), __fadd_rn(a.w, b.w));
+}
+__device__ __forceinline__ float4 mul4(float4 a, float b)
+{
+    return make_float4(__fmul_rn(a.x, b), __fmul_rn(a.y, b), __fmul_rn(a.z, b), __fmul_rn(a.w, b));
 }
 __device__ __forceinline__ float4 lerp4(float4 a, float4 b, float wa, float wb)
 {
@@ -129,6 +140,42 @@ struct SciWords {
         c[2] = keep > 2u ? (double)__fmul_rn(byte_to_float(r0, 3u), __ldg(scales + 1)) : 0.0;
         c[3] = keep > 3u ? (double)__fmul_rn(byte_to_float(r1, 0u), __ldg(scales + 2)) : 0.0;
     }
+    // Two controls (records at bytes ca and cb) at four frames f[0..3], any number of coefficients: the sum of
+    // sci_control, term by term, with a word of four coefficients, their scales and four basis values of each
+    // frame read at a time.
+    __device__ __forceinline__ void sums(uint32_t ca, uint32_t cb, uint32_t keep, const float* __restrict__ scales,
+                                         const float* __restrict__ basis, const int f[kSciWideFrames],
+                                         double sa[kSciWideFrames], double sb[kSciWideFrames]) const
+    {
+        const double da = (double)half_to_float_exact(u32(ca) & 0xFFFFu), db = (double)half_to_float_exact(u32(cb) & 0xFFFFu);
+#pragma unroll 1
+        for (uint32_t k0 = 0; k0 < keep; k0 += 4u) {
+            const uint32_t wa = u32(ca + 1u + k0), wb = u32(cb + 1u + k0);   // coefficient k is byte k + 1 of the record
+            float4 b[kSciWideFrames];
+#pragma unroll
+            for (int j = 0; j < kSciWideFrames; ++j)
+                b[j] = __ldg(reinterpret_cast<const float4*>(basis + (uint64_t)(uint32_t)f[j] * 64u + k0));
+#pragma unroll
+            for (uint32_t i = 0; i < 4u; ++i) {
+                if (k0 + i >= keep) break;
+                const bool dc = k0 + i == 0u;
+                const float sc = dc ? 0.0f : __ldg(scales + k0 + i - 1u);
+                const double qa = dc ? da : (double)__fmul_rn(byte_to_float(wa, i), sc);
+                const double qb = dc ? db : (double)__fmul_rn(byte_to_float(wb, i), sc);
+#pragma unroll
+                for (int j = 0; j < kSciWideFrames; ++j) {
+                    const double v = (double)(i == 0u ? b[j].x : i == 1u ? b[j].y : i == 2u ? b[j].z : b[j].w);
+                    sa[j] = dc ? qa * v : __fma_rn(qa, v, sa[j]);
+                    sb[j] = dc ? qb * v : __fma_rn(qb, v, sb[j]);
+                }
+            }
+        }
+    }
+    // sample ci of the BFP grid whose codes start at byte `data` (bfp_sample: at most two bytes of a code)
+    __device__ __forceinline__ uint32_t code(uint32_t data, uint32_t bit) const
+    {
+        return (u32(data + (bit >> 3)) & 0xFFFFu) >> (bit & 7u);
+    }
     // event i of a SparseEvents leaf whose keys start at word kw: key, and residual q * es
     __device__ __forceinline__ uint32_t event_key(uint32_t kw, uint32_t i) const
     {
@@ -142,24 +189,27 @@ struct SciWords {
     }
 };
 
-// Is the leaf of the common shape?  At most four coefficients per control; no events, or events
-// that the visit of a bin finds as the search does (kFlagSorted); no temporal-basis residual; every
-// section inside the payload.
+// Is the leaf of the common shape?  No events, or events that the visit of a bin finds as the search does
+// (kFlagSorted); every section inside the payload; and, but for the WIDE kernel, at most four coefficients per
+// control, no temporal-basis residual and codes of at most eight bits.
+template <bool WIDE>
 __device__ __forceinline__ bool sci_common_shape(const AssetGeom& g, const LeafEntry& e)
 {
     const uint64_t room = 4ull * (g.payload_words - e.word_off);
     const uint32_t hdr = e.header, mode = hdr & 3u, keep = ((hdr >> 2) & 0x3Fu) + 1u;
     const uint64_t sb = 4u + 64u * (keep + 1u);
-    if (keep > 4u || sb + 4u > room) return false;
+    if ((!WIDE && keep > 4u) || sb + 4u > room) return false;
     if (mode == 1u && ((hdr >> 16) & 0x0FFFu) != 0u) {
         const uint32_t tier = (hdr >> 8) & 3u;
         const uint32_t cap = tier == 0u ? 64u : tier == 1u ? 256u : tier == 2u ? 768u : 1024u;
         return (e.info & kFlagSorted) != 0u && sb + 100u + 2u * cap + cap / 2u <= room;
     }
     if (mode >= 2u) {
+        const bool tb = ((hdr >> 12) & 7u) == 1u;
         const uint32_t per = mode == 2u ? 27u : 64u, bits = (hdr >> 8) & 0xFu;
-        const uint64_t end = sb + 2ull * g.frames + (uint64_t)g.frames * ((per * bits + 7u) / 8u);
-        return ((hdr >> 12) & 7u) != 1u && bits <= 8u && end <= room && end < (1ull << 32);
+        const uint64_t grids = tb ? ((hdr >> 15) & 0xFu) + 1u : g.frames;
+        const uint64_t end = sb + grids * (2u + (per * bits + 7u) / 8u);
+        return (WIDE || (!tb && bits <= 8u)) && end <= room && end < (1ull << 32);
     }
     return true;
 }
@@ -167,19 +217,26 @@ __device__ __forceinline__ bool sci_common_shape(const AssetGeom& g, const LeafE
 // grid.x: one warp per leaf, so that the warps of a CTA write neighbouring leaves together (warps that
 // stride over leaves drift apart, and partly written lines fall out of L2: 64 dense frames of
 // 256 x 128 x 128 took 650 us instead of 380); grid.y: the chunks of the launch's frames in turn.
-// Leaves of no common shape (five or more coefficients, sections that leave the payload, unsorted
-// events, temporal-basis residuals) go through the per-frame functions.
+// Leaves of no common shape (sections that leave the payload, unsorted events) go through the per-frame
+// functions.
+// WIDE: for files with leaves of five or more coefficients, temporal-basis residuals or codes of over eight
+// bits (AssetGeom::wide).  Controls are summed four frames at a time from the payload instead of from four
+// registers; a temporal-basis residual keeps its decoded grids in shared memory and takes each one's
+// trilinear, which no frame changes, once for two frames.  Bound by instruction issue as the other.  64 frames
+// of 128^3 into the cache on a B200: 6 coefficients 206 us, 12 226, residuals of 8 basis grids 476 (leaf by leaf
+// and frame by frame 1,221, 1,467 and 4,348).  An instantiation of its own, since its controls and sums cost
+// the other kernel registers.
 // Four CTAs of 128 registers: with 96 registers and five, the spills and the wider spread of the writes
 // cost more than the warps hide (222 against 265 us).
 // LOOSE: a cache that starts at any float, its frames any number of floats apart (an instantiation of its
 // own: the test in the one kernel costs an aligned window of 64 frames of 128^3 1.5 %).
-template <bool DENSE, bool LOOSE>
+template <bool DENSE, bool LOOSE, bool WIDE>
 __global__ void __launch_bounds__(kSciWarps * 32, 4) sci_frames_kernel(DeviceAsset a, FrameList fl, int chunk,
                                                                        float* __restrict__ out, uint64_t frame_stride)
 {
-    __shared__ SciWarpShared s_all[kSciWarps];
+    __shared__ SciWarpShared<WIDE> s_all[kSciWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    SciWarpShared& sh = s_all[warp];
+    SciWarpShared<WIDE>& sh = s_all[warp];
     const uint32_t n_leaves = DENSE ? a.g.leaf_count : *(volatile const uint32_t*)a.counters;
     const int ly = (lane >> 1) & 7, lx0 = 4 * (lane & 1);
     const bool hz = lane >= 16;
@@ -245,7 +302,7 @@ __global__ void __launch_bounds__(kSciWarps * 32, 4) sci_frames_kernel(DeviceAss
         }
         if (lane < n) sh.frames[lane] = clamp_frame(fl.f[f0 + lane], (int)a.g.frames);
         __syncwarp();
-        if (!sci_common_shape(a.g, e)) {
+        if (!sci_common_shape<WIDE>(a.g, e)) {
             bool oob = false;
             for (int j = 0; j < n; ++j) {
                 const uint32_t t = (uint32_t)sh.frames[j];
@@ -268,10 +325,13 @@ __global__ void __launch_bounds__(kSciWarps * 32, 4) sci_frames_kernel(DeviceAss
         const SciWords lw{a.payload + e.word_off, room < 0x40000000ull ? (uint32_t)room : 0x40000000u};
         const uint32_t sb = 4u + 64u * (keep + 1u), sw = sb >> 2;
         // coefficients of controls lane and lane + 32, and the basis rows of the frames
+        const uint32_t cb0 = 4u + (uint32_t)lane * (keep + 1u), cb1 = cb0 + 32u * (keep + 1u);
         double c0[4], c1[4];
-        lw.coefficients(4u + (uint32_t)lane * (keep + 1u), keep, a.scales, c0);
-        lw.coefficients(4u + (uint32_t)(lane + 32) * (keep + 1u), keep, a.scales, c1);
-        for (int i = lane; i < n * 4; i += 32)
+        if constexpr (!WIDE) {
+            lw.coefficients(cb0, keep, a.scales, c0);
+            lw.coefficients(cb1, keep, a.scales, c1);
+        }
+        for (int i = lane; !WIDE && i < n * 4; i += 32)
             sh.basis[i >> 2][i & 3] = (double)__ldg(a.basis + (uint64_t)(uint32_t)sh.frames[i >> 2] * 64u + (uint32_t)(i & 3));
         // events of the item's time bins: each lane keeps two of them (64 in all; a 16-frame item of a
         // field with 0.5 % of its values stored as events has about 40), the others are read per frame
@@ -314,25 +374,96 @@ __global__ void __launch_bounds__(kSciWarps * 32, 4) sci_frames_kernel(DeviceAss
         uint32_t g0 = 0, g1 = 0, gs = 0;
         auto read_grid = [&](uint32_t t) {
             const uint32_t data = sb + 2u * a.g.frames + t * fbytes;
-            g0 = lw.u32(data + (gb0 >> 3)) >> (gb0 & 7u);
-            g1 = lw.u32(data + (gb1 >> 3)) >> (gb1 & 7u);
+            g0 = WIDE ? lw.code(data, gb0) : lw.u32(data + (gb0 >> 3)) >> (gb0 & 7u);
+            g1 = WIDE ? lw.code(data, gb1) : lw.u32(data + (gb1 >> 3)) >> (gb1 & 7u);
             gs = lw.u32(sb + 2u * t) & 0xFFFFu;
         };
-        if (mode >= 2u) read_grid((uint32_t)sh.frames[0]);
+        const bool tb = WIDE && mode >= 2u && ((hdr >> 12) & 7u) == 1u;   // the leaf's grids times basis values
+        if (mode >= 2u && !tb) read_grid((uint32_t)sh.frames[0]);
         // a code's level, by lane: the division of decode_bfp once per item (up to 5 bits)
         const float level = mode >= 2u ? decode_bfp((uint32_t)lane, 1.0f, (int)bits) : 0.0f;
+        // the controls of frames j .. j + 3, where j is the first of them
+        auto controls = [&](int j) {
+            int f[kSciWideFrames];
+            double sa[kSciWideFrames], sb2[kSciWideFrames];
+#pragma unroll
+            for (int i = 0; i < kSciWideFrames; ++i) f[i] = sh.frames[min(j + i, n - 1)];
+            lw.sums(cb0, cb1, keep, a.scales, a.basis, f, sa, sb2);
+#pragma unroll
+            for (int i = 0; i < kSciWideFrames; ++i) {
+                sh.ctrl[64 * i + lane] = (float)sa[i];
+                sh.ctrl[64 * i + 32 + lane] = (float)sb2[i];
+            }
+        };
+        if constexpr (WIDE) {
+            if (tb) {
+                const uint32_t tkeep = ((hdr >> 15) & 0xFu) + 1u, grids = bits ? tkeep : 0u;   // no bits: no residual
+                const uint32_t mask = (1u << bits) - 1u;
+                for (uint32_t i = (uint32_t)lane; i < grids * per; i += 32u) {
+                    const uint32_t k = i / per, ci = i - k * per;
+                    const float sc = half_to_float_exact(lw.u32(sb + 2u * k) & 0xFFFFu);
+                    sh.residual[64u * k + (mode == 2u ? ci / 3u * 4u + ci % 3u : ci)] =
+                        decode_bfp(lw.code(sb + 2u * tkeep + k * fbytes, ci * bits) & mask, sc, (int)bits);
+                }
+                const SciWeights<3> W3(lane);
+                __syncwarp();
+                for (int j = 0; j < n; j += 2) {
+                    if (j % kSciWideFrames == 0) controls(j);
+                    const float* r0 = a.basis + (uint64_t)(uint32_t)sh.frames[j] * 64u;
+                    const float* r1 = a.basis + (uint64_t)(uint32_t)sh.frames[min(j + 1, n - 1)] * 64u;
+                    float4 sum[2][4], q[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) sum[0][i] = sum[1][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    __syncwarp();
+#pragma unroll 1
+                    for (uint32_t k = 0; k < grids; ++k) {
+                        if (mode == 3u) sci_quads<4>(W, sh.residual + 64u * k, sh.x, lane, q);
+                        else sci_quads<3>(W3, sh.residual + 64u * k, sh.x, lane, q);
+                        const float b0 = __ldg(r0 + k), b1 = __ldg(r1 + k);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            sum[0][i] = add4(sum[0][i], mul4(q[i], b0));
+                            sum[1][i] = add4(sum[1][i], mul4(q[i], b1));
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        if (j + u >= n) break;
+                        sci_quads<4>(W, sh.ctrl + 64 * ((j + u) % kSciWideFrames), sh.x, lane, q);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) q[i] = add4(q[i], sum[u][i]);
+                        if (plain) {
+                            float* o = dst;
+#pragma unroll
+                            for (int i = 0; i < 4; ++i, o += zstep) __stcs(reinterpret_cast<float4*>(o), q[i]);
+                            dst += frame_stride;
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) put(j + u, ly, hz ? 7 - i : i, lx0, q[i]);
+                        }
+                    }
+                }
+                continue;
+            }
+        }
         __syncwarp();
         for (int j = 0; j < n; ++j) {
-            double s0 = c0[0] * sh.basis[j][0], s1 = c1[0] * sh.basis[j][0];
+            const float* ctrl = sh.ctrl;
+            if constexpr (WIDE) {
+                if (j % kSciWideFrames == 0) controls(j);
+                ctrl += 64 * (j % kSciWideFrames);
+            } else {
+                double s0 = c0[0] * sh.basis[j][0], s1 = c1[0] * sh.basis[j][0];
 #pragma unroll
-            for (int k = 1; k < 4; ++k)
-                if (k < (int)keep) {
-                    const double b = sh.basis[j][k];
-                    s0 = __fma_rn(c0[k], b, s0);
-                    s1 = __fma_rn(c1[k], b, s1);
-                }
-            sh.ctrl[lane] = (float)s0;
-            sh.ctrl[lane + 32] = (float)s1;
+                for (int k = 1; k < 4; ++k)
+                    if (k < (int)keep) {
+                        const double b = sh.basis[j][k];
+                        s0 = __fma_rn(c0[k], b, s0);
+                        s1 = __fma_rn(c1[k], b, s1);
+                    }
+                sh.ctrl[lane] = (float)s0;
+                sh.ctrl[lane + 32] = (float)s1;
+            }
             bool hit0 = false, hit1 = false;
             uint32_t code = 0u, r0 = 0u, r1 = 0u;   // the frame's bin, and its events that no lane keeps
             if (events) {
@@ -376,20 +507,17 @@ __global__ void __launch_bounds__(kSciWarps * 32, 4) sci_frames_kernel(DeviceAss
                     const SciWeights<3> W3(lane);
                     sci_quads<3>(W3, sh.residual, sh.x, lane, qr);
                 }
-                sci_quads<4>(W, sh.ctrl, sh.x, lane, q);
+                sci_quads<4>(W, ctrl, sh.x, lane, q);
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    q[i] = make_float4(__fadd_rn(q[i].x, qr[i].x), __fadd_rn(q[i].y, qr[i].y), __fadd_rn(q[i].z, qr[i].z),
-                                       __fadd_rn(q[i].w, qr[i].w));
+                for (int i = 0; i < 4; ++i) q[i] = add4(q[i], qr[i]);
             } else {
                 __syncwarp();
-                sci_quads<4>(W, sh.ctrl, sh.x, lane, q);
+                sci_quads<4>(W, ctrl, sh.x, lane, q);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     float4 r = make_float4(0.f, 0.f, 0.f, 0.f);   // a sum with +0 is not the value itself at -0
                     if (add) r = *reinterpret_cast<const float4*>(sh.residual + 64 * (hz ? 7 - i : i) + 8 * ly + lx0);
-                    q[i] = make_float4(__fadd_rn(q[i].x, r.x), __fadd_rn(q[i].y, r.y), __fadd_rn(q[i].z, r.z),
-                                       __fadd_rn(q[i].w, r.w));
+                    q[i] = add4(q[i], r);
                 }
             }
             if (plain) {
@@ -419,28 +547,39 @@ __global__ void __launch_bounds__(kSciWarps * 32, 4) sci_frames_kernel(DeviceAss
 // Frames per item: 16 where that leaves twelve or more items for every resident warp, else 8, and 4
 // where those would not give each warp two (an item's set-up costs about three frames; 64 frames of
 // 128^3: 8 frames per item 216 us, 16 235; of 256 x 128 x 128: 385 and 375).
-template <bool DENSE>
-static void launch_sci_frames(const DeviceAsset& a, const FrameList& fl, float* out, uint64_t stride, int grid,
-                              cudaStream_t s)
+template <bool DENSE, bool LOOSE, bool WIDE>
+static void launch_sci_variant(const DeviceAsset& a, const FrameList& fl, float* out, uint64_t stride, int grid,
+                               cudaStream_t s)
 {
     static int full = 0;
     if (!full) {
         int dev = 0, sms = 0, per = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sci_frames_kernel<DENSE, false>, kSciWarps * 32, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sci_frames_kernel<DENSE, LOOSE, WIDE>, kSciWarps * 32, 0);
         full = sms * (per > 0 ? per : 1);
     }
     const uint64_t warps = (uint64_t)full * kSciWarps, L = a.g.leaf_count;
     auto items = [&](int c) { return L * (uint64_t)((fl.n + c - 1) / c); };
     const int chunk = items(16) >= 12u * warps ? 16 : items(8) >= 2u * warps ? 8 : 4;
     const uint64_t most = (L + kSciWarps - 1) / kSciWarps;
-    const dim3 ctas((unsigned)(grid > 0 && (uint64_t)grid < most ? (uint64_t)grid : most),
-                    (unsigned)((fl.n + chunk - 1) / chunk));
-    if (!DENSE && ((stride & 3u) != 0u || (reinterpret_cast<uintptr_t>(out) & 15u) != 0u))
-        sci_frames_kernel<DENSE, !DENSE><<<ctas, kSciWarps * 32, 0, s>>>(a, fl, chunk, out, stride);
-    else
-        sci_frames_kernel<DENSE, false><<<ctas, kSciWarps * 32, 0, s>>>(a, fl, chunk, out, stride);
+    sci_frames_kernel<DENSE, LOOSE, WIDE><<<dim3((unsigned)(grid > 0 && (uint64_t)grid < most ? (uint64_t)grid : most),
+                                                 (unsigned)((fl.n + chunk - 1) / chunk)),
+                                            kSciWarps * 32, 0, s>>>(a, fl, chunk, out, stride);
+}
+
+template <bool DENSE>
+static void launch_sci_frames(const DeviceAsset& a, const FrameList& fl, float* out, uint64_t stride, int grid,
+                              cudaStream_t s)
+{
+    const bool loose = !DENSE && ((stride & 3u) != 0u || (reinterpret_cast<uintptr_t>(out) & 15u) != 0u);
+    if (a.g.wide) {
+        if (loose) launch_sci_variant<DENSE, !DENSE, true>(a, fl, out, stride, grid, s);
+        else launch_sci_variant<DENSE, false, true>(a, fl, out, stride, grid, s);
+    } else {
+        if (loose) launch_sci_variant<DENSE, !DENSE, false>(a, fl, out, stride, grid, s);
+        else launch_sci_variant<DENSE, false, false>(a, fl, out, stride, grid, s);
+    }
 }
 
 }  // namespace vbtb
