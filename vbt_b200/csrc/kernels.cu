@@ -732,11 +732,14 @@ __device__ __forceinline__ float sparse_at(SciReader& rd, const SparseLeaf& s, u
     const uint32_t bin = t / s.fpb < 15u ? t / s.fpb : 15u;
     const uint32_t lt = (t - bin * s.fpb) & 0xFFu;
     // inside the payload, the 16-bit fields are read as 32-bit windows (one or two word reads
-    // instead of two checked byte reads); the values are the same
-    auto u16 = [&](uint64_t b) { return s.inside ? (pay_u32(rd.pw, b) & 0xFFFFu) : rd.u16(b); };
+    // instead of two checked byte reads); the values are the same.  A bin of a bad file may reach past the
+    // section, and its keys past the payload: those are read checked.
+    bool inside = s.inside;
+    auto u16 = [&](uint64_t b) { return inside ? (pay_u32(rd.pw, b) & 0xFFFFu) : rd.u16(b); };
     const uint32_t start = u16(s.bb + bin * 2u);
     const uint32_t end = bin + 1u < 16u ? u16(s.bb + (bin + 1u) * 2u) : (s.count & 0xFFFFu);
     if (start >= end) return 0.0f;
+    inside = inside && end <= s.cap;
     const uint64_t cb = s.bb + 32u, rb = cb + s.cap * 2u;
     const uint32_t target = ((lt << 9) | (li & 0x1FFu)) & 0xFFFFu;
     int left = (int)start, right = (int)end - 1;
@@ -744,8 +747,7 @@ __device__ __forceinline__ float sparse_at(SciReader& rd, const SparseLeaf& s, u
         const int mid = (left + right) >> 1;
         const uint32_t key = u16(cb + (uint32_t)mid * 2u);
         if (key == target) {
-            const uint32_t byte = s.inside ? (pay_u32(rd.pw, rb + (uint32_t)(mid >> 1)) & 0xFFu)
-                                           : rd.byte(rb + (uint32_t)(mid >> 1));
+            const uint32_t byte = inside ? (pay_u32(rd.pw, rb + (uint32_t)(mid >> 1)) & 0xFFu) : rd.byte(rb + (uint32_t)(mid >> 1));
             int q = (int)((mid & 1) == 0 ? (byte & 0xFu) : ((byte >> 4) & 0xFu));
             if (q & 8) q -= 16;
             return __fmul_rn((float)q, s.es);
