@@ -21,11 +21,12 @@ namespace vbtb {
 // Eight CTAs per SM: 64 registers (some set-up values spill) and 32 warps, which hide the reads better
 // than 24 warps at 80 registers (fire 175 us); 40 warps at 48 gain on the fire (143) and lose on the
 // plume (74).
+// Events of a batch that eight lanes each look up in turn; more go to their own lanes.
+constexpr int kPqEvents = 8;
 constexpr int kPqWarps = 4, kPqCtas = 8, kPqThreads = 32 * kPqWarps, kPqBatch = 32;
 
 // The general decode of one scientific query (src: decodeScientificValueAtCpu,
-// render/src/scientific_decode.cpp:335-359) by one thread: leaves with more than seven coefficients
-// per control, sections that leave the payload, temporal-basis residual grids.
+// render/src/scientific_decode.cpp:335-359) by one thread: sections that leave the payload.
 __device__ __noinline__ float sci_point_general(const DeviceAsset& a, LeafEntry e, uint32_t lx, uint32_t ly, uint32_t lz,
                                                 uint32_t t, bool* oob_out)
 {
@@ -122,11 +123,76 @@ __device__ __forceinline__ float sci_event(const uint32_t* __restrict__ lw, uint
     return __fmul_rn((float)q, es);
 }
 
+// Axis weights of the common grids, [render 4^3, render 6^3, scientific 4^3, 3^3][position] = {t, i0}
+// (i1 is i0 + 1); a position inside a cropped leaf has the weights it has in a whole one.
+struct CellAxis {
+    uint32_t i0;
+    float t, omt;
+};
+
+// The same by one thread with the reference's search: keys in any order.  Also the events of a batch with many
+// of them: eight lanes to an event take a batch's events in turn, four at a time.
+__device__ __noinline__ float sci_event_alone(const DeviceAsset& a, LeafEntry e, uint32_t li, uint32_t t, bool* oob)
+{
+    SciReader rd{a.payload, a.g.payload_words, false};
+    const SparseLeaf sp = sparse_leaf(rd, 4ull * e.word_off, e.header, (int)((e.header >> 2) & 0x3Fu) + 1);
+    const float r = sp.es > 0.0f ? sparse_at(rd, sp, li, t) : 0.0f;
+    *oob = rd.oob;
+    return r;
+}
+
+// sci_control_fast for a record of any length.
+__device__ __noinline__ float sci_control_long(const uint32_t* __restrict__ w, uint32_t cb, uint32_t keep,
+                                               const float* __restrict__ brow, const float* __restrict__ scales)
+{
+    const uint32_t* p = w + (cb >> 2);
+    const uint32_t sh = (cb & 3u) * 8u;
+    uint32_t x = __ldg(p), y = __ldg(p + 1);
+    double sum = (double)half_to_float_exact(__funnelshift_r(x, y, sh) & 0xFFFFu) * (double)__ldg(brow);
+    for (uint32_t k0 = 0;; k0 += 4u) {   // record bytes k0 .. k0 + 3: the coefficients from k0 - 1 on
+        const uint32_t r = __funnelshift_r(x, y, sh);
+#pragma unroll
+        for (uint32_t i = 0; i < 4u; ++i) {
+            const uint32_t k = k0 + i - 1u;
+            if (k0 + i >= 2u && k < keep)
+                sum = __fma_rn((double)__fmul_rn(byte_to_float(r, i), __ldg(scales + k - 1u)), (double)__ldg(brow + k), sum);
+        }
+        if (k0 + 3u >= keep) return (float)sum;
+        x = y;
+        y = __ldg(p + 2u + (k0 >> 2));
+    }
+}
+
+// The temporal-basis residual of a query by eight lanes (`sub` = its corner of the cell, lane mask `mask`): of
+// each basis grid the lanes' samples, their trilinear by three exchanges, times the frame's basis value
+// (render/src/scientific_decode.cpp:177-233).  Codes of R^3 grids from byte `sb` of the leaf on.
+__device__ __noinline__ float sci_basis_residual(const uint32_t* __restrict__ lw, uint32_t sb, uint32_t hdr, uint32_t ci,
+                                                 CellAxis ax, CellAxis ay, CellAxis az,
+                                                 const float* __restrict__ brow, uint32_t sub, uint32_t mask)
+{
+    const uint32_t per = (hdr & 3u) == 2u ? 27u : 64u, bits = (hdr >> 8) & 0xFu, tkeep = ((hdr >> 15) & 0xFu) + 1u;
+    const uint32_t bo = ci * bits, bytes = (per * bits + 7u) / 8u;
+    float r = 0.0f;
+    for (uint32_t k = 0; bits != 0u && k < tkeep; ++k) {
+        const uint32_t code = ((pay_u32(lw, sb + 2u * tkeep + k * bytes + (bo >> 3)) & 0xFFFFu) >> (bo & 7u)) & ((1u << bits) - 1u);
+        float v = decode_bfp(code, half_to_float_exact(pay_u32(lw, sb + 2u * k) & 0xFFFFu), (int)bits);
+        auto along = [&](const CellAxis& w, uint32_t bit) {
+            const float o = __shfl_xor_sync(mask, v, (int)bit);
+            v = lerp_ref(sub & bit ? o : v, sub & bit ? v : o, w.t, w.omt);
+        };
+        along(ax, 1u);
+        along(ay, 2u);
+        along(az, 4u);
+        r = __fadd_rn(r, __fmul_rn(v, __ldg(brow + k)));
+    }
+    return r;
+}
+
 // What the corner step needs of a query.  Render leaves: `grids` = coarse corner 0 | R << 9 | fine
 // corner 0 << 12 | R << 21 | bin << 24 | sorted << 27 | FP32 codecs << 28, 29; `kf`, the fine
-// stream's byte offset in `at`, the frame in `t`.  Scientific leaves: corner 0 | keep << 9 |
-// residual corner 0 << 12 | residual R << 21, the header in `kf`, the residual grid's (or the event
-// section's) byte offset in `at`, the frame in `t`.
+// stream's byte offset in `at`, the frame in `t`.  Scientific leaves: corner 0 |
+// residual corner 0 << 12 | residual R << 21 | keep << 24, the header in `kf`, the residual grid's (or the event or
+// temporal-basis section's) byte offset in `at`, the frame in `t`.
 struct __align__(16) QueryCell {
     const uint32_t* lw;    // the leaf block
     const float* brow;     // scientific: basis row of the frame
@@ -136,17 +202,11 @@ struct __align__(16) QueryCell {
 
 struct QueryShared {
     QueryCell cell[kPqBatch];
-    float val[kPqBatch * 17];   // per query: 8 corners, 8 of the second grid, the event
+    float val[kPqBatch * 17];   // per query: 8 corners, 8 of the second grid, the event or temporal-basis residual
     uint16_t list[2 * kPqBatch];
-    uint8_t second[kPqBatch], events[kPqBatch];
+    uint8_t second[kPqBatch], residuals[kPqBatch];
 };
 
-// Axis weights of the common grids, [render 4^3, render 6^3, scientific 4^3, 3^3][position] = {t, i0}
-// (i1 is i0 + 1); a position inside a cropped leaf has the weights it has in a whole one.
-struct CellAxis {
-    uint32_t i0;
-    float t, omt;
-};
 __device__ __forceinline__ CellAxis cell_axis(const float2* table, int grid, uint32_t res, uint32_t pos)
 {
     float2 w;
@@ -192,7 +252,7 @@ __device__ __forceinline__ void query_batch(QueryShared& sh, const float2* table
     const uint32_t lane = threadIdx.x & 31u, sub = lane & 7u, group = lane >> 3, gmask = 0xFFu << (8u * group);
     enum : uint32_t { kNone, kRender, kSci, kSciGeneral };
     uint32_t kind = kNone, leaf = 0, place = 0;   // place: lx | ly << 3 | lz << 6
-    bool second = false, event = false;
+    bool second = false, event = false, alone = false, tbasis = false;
     const auto r = resolve.request(on ? i : 0);
     const DeviceAsset& a = resolve.asset(r);
     // 1. the lane's query
@@ -220,28 +280,33 @@ __device__ __forceinline__ void query_batch(QueryShared& sh, const float2* table
                 const uint32_t lim = room < 0xFFFFFFFFull ? (uint32_t)room : 0xFFFFFFFFu;
                 const uint32_t hdr = e.header, mode = hdr & 3u, keep = ((hdr >> 2) & 0x3Fu) + 1u;
                 const uint32_t sb = 4u + 64u * (keep + 1u);
-                bool plain = keep <= 7u && sb + 4u <= lim;
+                bool plain = sb + 4u <= lim;
                 c.brow = a.basis + (uint64_t)t * 64u;
                 c.scales = a.scales;
-                c.grids = cell_corner(table, 2, 4u, lx, ly, lz) | (keep << 9);
+                c.grids = cell_corner(table, 2, 4u, lx, ly, lz) | (keep << 24);
                 c.kf = hdr;
                 c.t = t;
                 c.voxel = (lz * 8u + ly) * 8u + lx;
                 if (mode == 1u && ((hdr >> 16) & 0x0FFFu) != 0u) {
                     const uint32_t tier = (hdr >> 8) & 3u;
                     const uint32_t cap = tier == 0u ? 64u : tier == 1u ? 256u : tier == 2u ? 768u : 1024u;
-                    plain = plain && (e.info & kFlagSorted) != 0u && sb + 100u + 2u * cap + cap / 2u <= lim;
+                    plain = plain && sb + 100u + 2u * cap + cap / 2u <= lim;
+                    alone = (e.info & kFlagSorted) == 0u;
                     c.at = sb;
                     c.scale = cap;
                     event = plain && ((__ldg(c.lw + (sb >> 2) + 1u + (c.voxel >> 5)) >> (c.voxel & 31u)) & 1u) != 0u;
                 } else if (mode >= 2u) {
                     const uint32_t res = mode == 2u ? 3u : 4u, bits = (hdr >> 8) & 0xFu;
-                    const uint64_t data = (uint64_t)sb + 2ull * a.g.frames + (uint64_t)t * ((res * res * res * bits + 7u) / 8u);
-                    plain = plain && ((hdr >> 12) & 7u) != 1u && bits <= 8u && data + 4u + res * res * res <= lim;
-                    c.at = (uint32_t)data;
+                    const uint32_t bytes = (res * res * res * bits + 7u) / 8u;
+                    tbasis = ((hdr >> 12) & 7u) == 1u;
+                    const uint32_t grids = tbasis ? ((hdr >> 15) & 0xFu) + 1u : a.g.frames;
+                    const uint64_t data = (uint64_t)sb + 2ull * grids + (tbasis ? 0ull : (uint64_t)t * bytes);
+                    plain = plain && data + (tbasis ? (uint64_t)grids : 1ull) * bytes <= lim;
+                    c.at = tbasis ? sb : (uint32_t)data;
                     c.scale = sb + 2u * t;
                     c.grids |= (cell_corner(table, mode == 2u ? 3 : 2, res, lx, ly, lz) << 12) | (res << 21);
-                    second = plain;
+                    second = plain && !tbasis;
+                    tbasis = plain && tbasis;
                 }
                 kind = plain ? kSci : kSciGeneral;
             }
@@ -266,12 +331,17 @@ __device__ __forceinline__ void query_batch(QueryShared& sh, const float2* table
         sh.cell[lane] = c;
     }
     const uint32_t m1 = __ballot_sync(0xFFFFFFFFu, kind == kRender || kind == kSci);
-    const uint32_t m2 = __ballot_sync(0xFFFFFFFFu, second), m3 = __ballot_sync(0xFFFFFFFFu, event);
+    const uint32_t m2 = __ballot_sync(0xFFFFFFFFu, second);
+    // a batch's events: eight lanes to each, or, when they are many, each lane its own
+    const uint32_t me = __ballot_sync(0xFFFFFFFFu, event);
+    alone = alone || __popc(me) > kPqEvents;
+    const bool residual = tbasis || (event && !alone);
+    const uint32_t m3 = __ballot_sync(0xFFFFFFFFu, residual);
     const uint32_t below = (1u << lane) - 1u;
     const bool sci = a.g.profile == 2u;
     const uint32_t msci = __ballot_sync(0xFFFFFFFFu, on && sci);
     if (second) sh.second[__popc(m2 & below)] = (uint8_t)lane;
-    if (event) sh.events[__popc(m3 & below)] = (uint8_t)lane;
+    if (residual) sh.residuals[__popc(m3 & below)] = (uint8_t)lane;
     __syncwarp();
     // 2. the corners: four queries at a time
     for (uint32_t s0 = 0; s0 < batch; s0 += 4u) {
@@ -281,8 +351,9 @@ __device__ __forceinline__ void query_batch(QueryShared& sh, const float2* table
         const uint32_t g = c.grids;
         float v = 0.0f;
         if ((msci >> s) & 1u) {
-            const uint32_t keep = (g >> 9) & 7u;
-            v = sci_control_fast(c.lw, 4u + ((g & 0x1FFu) + corner_step(sub, 4u)) * (keep + 1u), (int)keep, c.brow, c.scales);
+            const uint32_t keep = g >> 24, cb = 4u + ((g & 0x1FFu) + corner_step(sub, 4u)) * (keep + 1u);
+            v = keep <= 7u ? sci_control_fast(c.lw, cb, (int)keep, c.brow, c.scales)
+                           : sci_control_long(c.lw, cb, keep, c.brow, c.scales);
         } else {
             const uint32_t R = (g >> 9) & 7u;
             if (R != 0u)
@@ -299,7 +370,7 @@ __device__ __forceinline__ void query_batch(QueryShared& sh, const float2* table
         float v = 0.0f;
         if ((msci >> s) & 1u) {   // bfp_sample at bit ci * bits of the frame's grid
             const uint32_t bits = (c.kf >> 8) & 0xFu, bo = ci * bits;
-            const uint32_t code = (pay_u32(c.lw, c.at + (bo >> 3)) >> (bo & 7u)) & ((1u << bits) - 1u);
+            const uint32_t code = ((pay_u32(c.lw, c.at + (bo >> 3)) & 0xFFFFu) >> (bo & 7u)) & ((1u << bits) - 1u);
             v = decode_bfp(code, half_to_float_exact(pay_u32(c.lw, c.scale) & 0xFFFFu), (int)bits);
         } else if (R != 0u) {
             v = control_at(LeafStream{c.lw, c.at, R * R * R, 8u, c.kf >> 16}, (g >> 29) & 1u, ci, (int)c.t,
@@ -308,9 +379,18 @@ __device__ __forceinline__ void query_batch(QueryShared& sh, const float2* table
         sh.val[s * 17u + 8u + sub] = v;
     }
     for (uint32_t k = group; k < n3; k += 4u) {
-        const uint32_t s = sh.events[k];
+        const uint32_t s = sh.residuals[k];
         const QueryCell& c = sh.cell[s];
-        const float v = sci_event(c.lw, c.at, c.kf, c.scale, c.voxel, c.t, sub, gmask);
+        float v;
+        if ((c.kf & 3u) == 1u) {
+            v = sci_event(c.lw, c.at, c.kf, c.scale, c.voxel, c.t, sub, gmask);
+        } else {
+            const uint32_t R = (c.grids >> 21) & 7u;
+            const int grid = R == 3u ? 3 : 2;
+            v = sci_basis_residual(c.lw, c.at, c.kf, ((c.grids >> 12) & 0x1FFu) + corner_step(sub, R),
+                                   cell_axis(table, grid, R, c.voxel & 7u), cell_axis(table, grid, R, (c.voxel >> 3) & 7u),
+                                   cell_axis(table, grid, R, c.voxel >> 6), c.brow, sub, gmask);
+        }
         if (sub == 0u) sh.val[s * 17u + 16u] = v;
     }
     __syncwarp();
@@ -344,7 +424,12 @@ __device__ __forceinline__ void query_batch(QueryShared& sh, const float2* table
             if ((e.info & kFlagOccClamp) && !in_occ && out < 0.0f) out = 0.0f;
         } else if (kind == kSci) {
             const float coarse = cell_value(table, 2, 4u, lx, ly, lz, v);
-            float res = event ? v[16] : 0.0f;
+            float res = residual ? v[16] : 0.0f;
+            if (event && alone) {
+                bool oob = false;
+                res = sci_event_alone(a, a.entries[leaf], (lz * 8u + ly) * 8u + lx, sh.cell[lane].t, &oob);
+                if (oob) record_error(resolve.err(r), leaf, kErrDecodeOob);
+            }
             if (second) res = (sh.cell[lane].kf & 3u) == 2u ? cell_value(table, 3, 3u, lx, ly, lz, v + 8)
                                                     : cell_value(table, 2, 4u, lx, ly, lz, v + 8);
             out = __fadd_rn(coarse, res);
