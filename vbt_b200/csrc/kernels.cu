@@ -1121,6 +1121,36 @@ void launch_decode_cache_plain(const DeviceAsset& a, int frame, float* out, cuda
 #include "point_query.cuh"
 namespace vbtb {
 
+// One voxel of a scientific leaf from the controls of sci_decode_controls, as sci_row makes it: a layer's 64
+// voxels are two per lane (a row of eight per lane left 24 lanes idle; 16 frames of a layer of 128 x 128 with
+// 3^3 residual grids, the call: 31 us so, 15 here).
+__device__ __forceinline__ float sci_voxel(const DeviceAsset& a, const LeafEntry& e, const float* __restrict__ s_ctrl,
+                                           uint32_t t, int lx, int ly, int lz, bool& oob)
+{
+    const uint32_t hdr = e.header, mode = hdr & 3u;
+    const float coarse = tri_small(s_ctrl, 4, g_sci_axis[0][lx], g_sci_axis[0][ly], g_sci_axis[0][lz]);
+    float r = 0.0f;
+    if (mode == 1u) {
+        SciReader rd{a.payload, a.g.payload_words, false};
+        const SparseLeaf sp = sparse_leaf(rd, 4ull * e.word_off, hdr, (int)((hdr >> 2) & 0x3Fu) + 1);
+        const uint32_t li = (uint32_t)((lz * 8 + ly) * 8 + lx);
+        if (sp.count && sp.es > 0.0f && ((sparse_mask_word(rd, sp, li >> 5) >> (li & 31u)) & 1u)) r = sparse_at(rd, sp, li, t);
+        oob |= rd.oob;
+    } else if (mode >= 2u) {
+        const int res = mode == 2u ? 3 : 4, g = mode == 2u ? 1 : 2, per = res * res * res;
+        auto tri = [&](const float* s) { return tri_small(s, res, g_sci_axis[g][lx], g_sci_axis[g][ly], g_sci_axis[g][lz]); };
+        if (((hdr >> 12) & 7u) == 1u) {
+            const int tkeep = (int)((hdr >> 15) & 0xFu) + 1;
+            const float* brow = a.basis + (uint64_t)t * 64u;
+            for (int k = 0; ((hdr >> 8) & 0xFu) != 0u && k < tkeep; ++k)
+                r = __fadd_rn(r, __fmul_rn(tri(s_ctrl + 64 + k * per), __ldg(brow + k)));
+        } else {
+            r = tri(s_ctrl + 64);
+        }
+    }
+    return __fadd_rn(coarse, r);
+}
+
 // Rows of one leaf of a z layer at frame t, by a warp: `dst` is the layer's row 0 at the leaf's first
 // voxel (zeros for EMPTY leaves, failed ones and frames of a scientific asset out of range).
 __device__ __forceinline__ void slice_tile(const DeviceAsset& a, uint32_t leaf, uint32_t z, int t, float* __restrict__ dst,
@@ -1149,11 +1179,9 @@ __device__ __forceinline__ void slice_tile(const DeviceAsset& a, uint32_t leaf, 
     bool oob = false;
     sci_decode_controls(a, e, (uint32_t)t, sm, lane, oob);
     __syncwarp();
-    if (lane < 8) {
-        float v[8];
-        sci_row(a, e, sm, (uint32_t)t, w, h, d, lane, lz, v, oob);
-        put(lane, 0, make_float4(v[0], v[1], v[2], v[3]));
-        put(lane, 4, make_float4(v[4], v[5], v[6], v[7]));
+    for (int i = lane; i < 64; i += 32) {
+        const int ly = i >> 3, lx = i & 7;
+        if (ly < h && lx < w) dst[(uint64_t)((uint32_t)ly) * a.g.width + (uint32_t)lx] = sci_voxel(a, e, sm, (uint32_t)t, lx, ly, lz, oob);
     }
     if (__any_sync(0xFFFFFFFFu, oob) && lane == 0) record_error(err, leaf, kErrDecodeOob);
     __syncwarp();
