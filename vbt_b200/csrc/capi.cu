@@ -169,6 +169,8 @@ int set_last_error(int status, const std::string& msg) { return fail(status, msg
 // Render-temporal:
 //  - sparse: fewer than half of the leaves non-EMPTY (the point-query kernel's shape hint);
 //  - mode2: a Mode2 leaf among them;
+//  - few_frames: the few-frames rule (kFewFrames, kernels.cuh), by the share of non-EMPTY leaves with FP16 keys
+//    and the grids that its kernel is made for;
 //  - the shared-memory leaf stage of the render decode kernel: the largest 16-byte-aligned window
 //    of a non-EMPTY leaf, capped so that two CTAs fit on an SM (232,448 B of shared memory per SM
 //    less 1 KiB per CTA); an asset with bigger leaves gets the kernel variant that decodes those
@@ -191,14 +193,16 @@ static void image_shape(const vbt_header& h, const uint8_t* b, uint64_t off_off,
         return;
     }
     const uint32_t cap = ((233472u / 2u - 1024u - kLeafFixedBytes - 16u) / 1024u) * 1024u;
-    uint64_t active = 0, maxw = 0, fits = 0, mode2 = 0;
+    uint64_t active = 0, maxw = 0, fits = 0, mode2 = 0, common = 0;
     for (uint32_t i = 0; i < h.leaf_count; ++i) {
         const uint64_t w0 = rd32(off + 4ull * i), w1 = rd32(off + 4ull * (i + 1));
         if (w1 <= w0 || w0 >= words) continue;
-        const uint32_t mode = rd32(b + pay_off + 4ull * w0) & 3u;
+        const uint32_t hdr = rd32(b + pay_off + 4ull * w0), mode = hdr & 3u;
         if (mode == kModeEmpty) continue;
         ++active;
         mode2 += mode == kModeFineCompact ? 1u : 0u;
+        const bool second = mode == kModeGrid4 || ((hdr >> 4) & 3u) != 1u;   // no second stream, or FP16 keys in it
+        common += ((hdr >> 6) & 7u) == 4u && ((hdr >> 2) & 3u) != 1u && second && (mode != kModeFine6 || ((hdr >> 9) & 7u) == 6u);
         const uint64_t a0 = (4ull * w0) & ~15ull, a1 = (4ull * w1 + 15u) & ~15ull;
         maxw = std::max(maxw, a1 - a0);
         fits += a1 - a0 <= cap ? 1u : 0u;
@@ -206,6 +210,7 @@ static void image_shape(const vbt_header& h, const uint8_t* b, uint64_t off_off,
     sparse = 2u * active < (uint64_t)h.leaf_count;
     g.sparse = sparse ? 1u : 0u;
     g.mode2 = mode2 != 0 ? 1u : 0u;
+    g.few_frames = 4u * common >= 3u * active ? kFewFrames : kFewFramesGeneral;
     g.max_window = (uint32_t)std::min<uint64_t>(maxw, 0xFFFFFFFFull);
     g.stage_bytes = std::min<uint32_t>(std::max<uint32_t>((g.max_window + 1023u) & ~1023u, 4096u), cap);
     if (4u * fits < 3u * active) g.stage_bytes = 0u;

@@ -492,10 +492,12 @@ __device__ __forceinline__ void rt_decode_controls(const DeviceAsset& a, const L
     }
 }
 
-// Reconstruct one row (ly, lz) of 8 voxels from the decoded controls.  Voxels outside the leaf
-// extent come out as 0 (they are not part of the frame; in the cache they are defined as 0).
-__device__ __forceinline__ void rt_row(const DeviceAsset& a, const LeafEntry& e, const float* __restrict__ s_ctrl,
-                                       int w, int h, int d, int ly, int lz, float out[8])
+// Reconstruct N voxels from lx0 on of row (ly, lz) from the decoded controls.  Voxels outside the leaf
+// extent come out as 0 (they are not part of the frame; in the cache they are defined as 0).  A row's x weights
+// are the same for all lanes and come from constant memory, those of a part differ.
+template <int N>
+__device__ __forceinline__ void rt_voxels(const DeviceAsset& a, const LeafEntry& e, const float* __restrict__ s_ctrl,
+                                          int w, int h, int d, int lx0, int ly, int lz, float out[N])
 {
     const uint32_t cres = (e.header >> 6) & 7u, fres = (e.header >> 9) & 7u;
     const AxisWeight ay = g_axis[axis_index(cres, h, ly)], az = g_axis[axis_index(cres, d, lz)];
@@ -518,22 +520,30 @@ __device__ __forceinline__ void rt_row(const DeviceAsset& a, const LeafEntry& e,
     }
     const bool shell = (e.info & kFlagShell) != 0u;
 #pragma unroll
-    for (int lx = 0; lx < 8; ++lx) {
+    for (int i = 0; i < N; ++i) {
+        const int lx = lx0 + i;
         float v = 0.0f;
         if (lx < w && ly < h && lz < d) {
-            v = trilinear_rt(s_ctrl, (int)cres, c_axis[axis_index(cres, w, lx)], ay, az);
+            v = trilinear_rt(s_ctrl, (int)cres, N == 8 ? c_axis[axis_index(cres, w, lx)] : g_axis[axis_index(cres, w, lx)], ay, az);
             const uint32_t bit = (uint32_t)(ly * 8 + lx);
             const bool in_occ = occ && ((mask >> bit) & 1ull);
             if (fine) {
-                v = __fadd_rn(v, trilinear_rt(s_ctrl + 343, (int)fres, c_axis[axis_index(fres, w, lx)], fy, fz));
+                v = __fadd_rn(v, trilinear_rt(s_ctrl + 343, (int)fres, N == 8 ? c_axis[axis_index(fres, w, lx)] : g_axis[axis_index(fres, w, lx)],
+                                              fy, fz));
             } else if (shell && in_occ) {
                 const uint32_t di = (pref + __popcll(mask & ((1ull << bit) - 1ull))) & 0xFFFFu;
                 v = __fadd_rn(v, s_ctrl[343 + di]);
             }
             if (occ && !in_occ && v < 0.0f) v = 0.0f;
         }
-        out[lx] = v;
+        out[i] = v;
     }
+}
+// The whole row.
+__device__ __forceinline__ void rt_row(const DeviceAsset& a, const LeafEntry& e, const float* __restrict__ s_ctrl,
+                                       int w, int h, int d, int ly, int lz, float out[8])
+{
+    rt_voxels<8>(a, e, s_ctrl, w, h, d, 0, ly, lz, out);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -969,12 +979,6 @@ namespace vbtb {
 #include "rt_frames.cuh"
 namespace vbtb {
 
-// Up to this many frames a launch reads the keys of each frame from the payload (rt_frames.cuh); more
-// are streamed from whole leaves in shared memory (rt_kernel_leaf.cuh).  Caches on a B200, read against
-// streamed: 6 frames of a 128 x 128 x 192 fire 89 / 112 us, of a 256^3 plume 81 / 94, of a 128^3 level
-// set 63 / 101; 8 frames 116 / 124, 107 / 102, 79 / 109; 16 frames 216 / 181, 194 / 141, 136 / 159.
-constexpr int kFewFrames = 6;
-
 void launch_decode_cache(const DeviceAsset& a, uint32_t seq, const int* frames, int nframes, float* out,
                          uint64_t stride, int grid, cudaStream_t s)
 {
@@ -983,7 +987,7 @@ void launch_decode_cache(const DeviceAsset& a, uint32_t seq, const int* frames, 
     for (int i = 0; i < nframes; ++i) fl.f[i] = frames[i];
     if (a.g.profile == 2u)
         launch_sci_frames<false>(a, fl, out, stride, grid, s);
-    else if (nframes <= kFewFrames && grid == 0)
+    else if (nframes <= (int)a.g.few_frames && grid == 0)
         launch_rt_frames<false>(a, fl, out, stride, 0, s);
     else
         launch_rt_leaf(a, seq, fl, out, stride, grid, false, s);
@@ -1055,7 +1059,7 @@ void launch_decode_dense(const DeviceAsset& a, uint32_t seq, const int* frames, 
     const uint64_t stride = (uint64_t)a.g.width * a.g.height * a.g.depth;
     if (a.g.profile == 2u)
         launch_sci_frames<true>(a, fl, out, stride, grid, s);
-    else if (nframes <= kFewFrames && grid == 0)
+    else if (nframes <= (int)a.g.few_frames && grid == 0)
         launch_rt_frames<true>(a, fl, out, stride, 0, s);
     else
         launch_rt_leaf(a, seq, fl, out, stride, grid, true, s);

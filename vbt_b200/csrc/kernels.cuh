@@ -17,6 +17,7 @@ struct AssetGeom {
     uint32_t max_window;    // largest 16-byte-aligned window of a non-EMPTY leaf
     uint32_t sparse;        // 1: render-temporal with most leaves EMPTY (the point-query shape)
     uint32_t mode2;         // 1: some leaf is a Mode2 one (the streaming kernel with its path)
+    uint32_t few_frames;    // render: launches of up to this many frames read each frame's keys (rt_frames.cuh)
     uint32_t wide;          // scientific, 1: leaves that need the WIDE frames kernel (sci_frames.cuh)
 };
 
@@ -44,6 +45,14 @@ constexpr uint32_t kWorkSlots = 64;
 
 // Frames of one decode launch (the frame list travels as a kernel parameter).
 constexpr int kMaxLaunchFrames = 128;
+
+// Up to this many frames a launch reads the keys of each frame from the payload (rt_frames.cuh); more
+// are streamed from whole leaves in shared memory (rt_kernel_leaf.cuh).  Caches on a B200, files not in L2, read
+// against streamed: 6 frames of a 128 x 128 x 192 fire 93 / 106 us, of a 256^3 plume 81 / 87, of a 128^3 level
+// set 69 / 79; 8 frames 118 / 115, 105 / 93, 85 / 86.
+// Leaves of other grids or with FP32 keys are read by the general functions, control by control: 2 frames of the
+// same fire with FP32 keys 122 / 161 us, 4 frames 221 / 168; with 5^3 grids 135 / 176, 238 / 186.
+constexpr uint32_t kFewFrames = 6, kFewFramesGeneral = 2;
 
 // Fixed shared memory of the render decode kernel besides its leaf stage (rt_kernel_leaf.cuh:
 // barrier, frame tables, axis weights, 9 warps x (x-lerp + y-lerp rows), 3072-float controls,

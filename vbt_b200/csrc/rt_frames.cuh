@@ -147,11 +147,10 @@ __device__ __forceinline__ void rt_leaf_layer(const DeviceAsset& a, const LeafEn
     if (!rt_common_shape(e)) {
         rt_decode_controls(a, e, frame, sm, lane);
         __syncwarp();
-        if (lane < 8) {
-            float v[8];
-            rt_row(a, e, sm, w, h, d, lane, lz, v);
-            put(lane, 0, make_float4(v[0], v[1], v[2], v[3]));
-            put(lane, 4, make_float4(v[4], v[5], v[6], v[7]));
+        if (lane < 16) {
+            float v[4];
+            rt_voxels<4>(a, e, sm, w, h, d, 4 * (lane & 1), lane >> 1, lz, v);
+            put(lane >> 1, 4 * (lane & 1), make_float4(v[0], v[1], v[2], v[3]));
         }
         __syncwarp();
         return;
