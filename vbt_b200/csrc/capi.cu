@@ -168,7 +168,8 @@ int set_last_error(int status, const std::string& msg) { return fail(status, msg
 //    eight bits (the frames kernel that covers them).
 // Render-temporal:
 //  - sparse: fewer than half of the leaves non-EMPTY (the point-query kernel's shape hint);
-//  - mode2: a Mode2 leaf among them;
+//  - mode2: a Mode2 leaf with FP16 keys and a 4^3 grid among them (the kernel with the specialised path for
+//    these);
 //  - few_frames: the few-frames rule (kFewFrames, kernels.cuh), by the share of non-EMPTY leaves with FP16 keys
 //    and the grids that its kernel is made for;
 //  - the shared-memory leaf stage of the render decode kernel: the largest 16-byte-aligned window
@@ -200,9 +201,10 @@ static void image_shape(const vbt_header& h, const uint8_t* b, uint64_t off_off,
         const uint32_t hdr = rd32(b + pay_off + 4ull * w0), mode = hdr & 3u;
         if (mode == kModeEmpty) continue;
         ++active;
-        mode2 += mode == kModeFineCompact ? 1u : 0u;
         const bool second = mode == kModeGrid4 || ((hdr >> 4) & 3u) != 1u;   // no second stream, or FP16 keys in it
-        common += ((hdr >> 6) & 7u) == 4u && ((hdr >> 2) & 3u) != 1u && second && (mode != kModeFine6 || ((hdr >> 9) & 7u) == 6u);
+        const bool usual = ((hdr >> 6) & 7u) == 4u && ((hdr >> 2) & 3u) != 1u && second && (mode != kModeFine6 || ((hdr >> 9) & 7u) == 6u);
+        common += usual ? 1u : 0u;
+        mode2 += usual && mode == kModeFineCompact ? 1u : 0u;
         const uint64_t a0 = (4ull * w0) & ~15ull, a1 = (4ull * w1 + 15u) & ~15ull;
         maxw = std::max(maxw, a1 - a0);
         fits += a1 - a0 <= cap ? 1u : 0u;

@@ -16,7 +16,7 @@ struct AssetGeom {
     uint32_t stage_bytes;   // shared-memory leaf stage of the render decode kernel (0 = none)
     uint32_t max_window;    // largest 16-byte-aligned window of a non-EMPTY leaf
     uint32_t sparse;        // 1: render-temporal with most leaves EMPTY (the point-query shape)
-    uint32_t mode2;         // 1: some leaf is a Mode2 one (the streaming kernel with its path)
+    uint32_t mode2;         // 1: some Mode2 leaf is of the specialised path's kind (the streaming kernel with it)
     uint32_t few_frames;    // render: launches of up to this many frames read each frame's keys (rt_frames.cuh)
     uint32_t wide;          // scientific, 1: leaves that need the WIDE frames kernel (sci_frames.cuh)
 };

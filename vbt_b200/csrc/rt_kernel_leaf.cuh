@@ -129,7 +129,7 @@ struct QuadSink {
 // warps; each finished quad of 4 voxels goes to `sink(frame index, lz, ly, lx0, values)`.  Frame
 // lists that step by 0 or 1 stream each control's keys; other non-decreasing lists (`monotone`)
 // walk a cursor; anything else, or keys that do not strictly increase, uses the reference's search.
-template <class M, class Sink, int NW>
+template <class M, class Sink, int NW, bool SHELL>
 __device__ __forceinline__ void leaf_decode(const DeviceAsset& a, const M& m, const LeafSmem& s, const LeafEntry& e,
                                             int nframes, bool steps01, bool monotone, const LeafGeom& G,
                                             const Sink& sink)
@@ -156,9 +156,10 @@ __device__ __forceinline__ void leaf_decode(const DeviceAsset& a, const M& m, co
     const bool cursor = !stream && monotone && (e.info & kFlagSorted) != 0u;
     const bool plain = !occ && G.w == 8 && G.h == 8 && G.d == 8;
     const int ly = (lane >> 1) & 7, lx0 = 4 * (lane & 1);
-    // GRID4 and Mode2 leaves with 4^3 controls take the specialised path's trilinear, whose lanes hold
-    // layers i and 7 - i
-    const bool grid4 = cres == 4 && !fine;
+    // in the kernel for Mode2 files, GRID4 and Mode2 leaves with 4^3 controls take the specialised path's
+    // trilinear, whose lanes hold layers i and 7 - i; in the other, where few leaves come here, the choice costs
+    // the others more (5^3 grids, 32 frames: 520 us with it, 504 without)
+    const bool grid4 = SHELL && cres == 4 && !fine;
     auto layer = [&](int i) { return grid4 ? (lane >= 16 ? 7 - i : i) : 2 * i + (lane >> 4); };
     uint64_t mask[4] = {0, 0, 0, 0};
     uint32_t pref[4] = {0, 0, 0, 0};
@@ -331,15 +332,15 @@ __device__ __forceinline__ void zero_band(const DeviceAsset& a, float* __restric
 // cheap leaves (few controls, few keys) take more of them.
 // The general decode as a call of its own, so that its registers do not crowd the fast path's
 // (the kernel's shared-memory layout is recomputed from the dynamic shared-memory base).
-template <class M, bool DENSE>
+template <class M, bool DENSE, bool SHELL>
 __device__ __noinline__ void leaf_decode_general(const DeviceAsset& a, M m, LeafEntry e, int nframes, bool steps01,
                                                  bool monotone, LeafGeom G, float* __restrict__ out,
                                                  uint64_t frame_stride)
 {
     extern __shared__ __align__(128) uint8_t dyn[];
     const LeafSmem s = leaf_layout<kDecWarps>(dyn);
-    leaf_decode<M, FrameSink<DENSE>, kDecWarps>(a, m, s, e, nframes, steps01, monotone, G,
-                                                FrameSink<DENSE>{a, G, out, frame_stride});
+    leaf_decode<M, FrameSink<DENSE>, kDecWarps, SHELL>(a, m, s, e, nframes, steps01, monotone, G,
+                                                       FrameSink<DENSE>{a, G, out, frame_stride});
 }
 
 // The specialised decode (rt_leaf_fast.cuh) as a call of its own too: each path gets the whole
@@ -486,10 +487,10 @@ __global__ void __launch_bounds__(kDecThreads, 2) decode_leaf_kernel(const __gri
                 }
             } else if (staged) {
                 const SharedWords m{reinterpret_cast<const uint32_t*>(s.stage), (uint32_t)(a0 >> 2)};
-                leaf_decode_general<SharedWords, DENSE>(a, m, e, fl.n, steps01, monotone, G, out, frame_stride);
+                leaf_decode_general<SharedWords, DENSE, SHELL>(a, m, e, fl.n, steps01, monotone, G, out, frame_stride);
             } else if (GLOBAL_FALLBACK) {
                 const GlobalWords m{a.payload};
-                leaf_decode_general<GlobalWords, DENSE>(a, m, e, fl.n, steps01, monotone, G, out, frame_stride);
+                leaf_decode_general<GlobalWords, DENSE, SHELL>(a, m, e, fl.n, steps01, monotone, G, out, frame_stride);
             }
         }
         __syncthreads();   // the next index is visible
