@@ -360,8 +360,11 @@ int vbt_window_error(vbt_asset* asset, int t0, int n, const float* d_values, uin
  * (t - f0) / (f1 - f0) of src/render_temporal_decode.cpp:129-130 without a division: one
  * reciprocal per key interval and a Markstein correction per frame.  This compares that quotient
  * with IEEE division on `device` for every integer pair 0 < a < b <= b_max (b_max <= 65535, the
- * widest key-frame span).  result[0] = mismatches, result[1] = smallest failing (b << 16 | a), or
- * all ones when there is none.  Synchronous. */
+ * widest key-frame span), the quotient that single frames use (an approximate reciprocal, corrected) for
+ * every 0 <= a <= b <= 255, and the axis weights of the ray sampler's 4^3 and 6^3 grids with the shader's
+ * two divisions for every position and leaf extent that takes them.  result[0] = mismatches, result[1] =
+ * smallest failing (b << 16 | a), for an axis weight 2^63 | R << 40 | extent << 32 | position bits, or all
+ * ones when there is none.  Synchronous. */
 int vbt_selftest_key_division(uint32_t b_max, uint64_t* result, int device);
 
 /* ---- Batched timeline: autotuned, graph-captured ---------------------------------------------

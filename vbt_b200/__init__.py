@@ -514,8 +514,9 @@ def selftest_keyframe_division(b_max=1024, device=0):
 
 
 def selftest_key_division(b_max=65535, device=0):
-    """(mismatches, smallest failing b << 16 | a) of the render decode's division-free interval
-    quotient against IEEE division, over every 0 < a < b <= b_max."""
+    """(mismatches, smallest failing b << 16 | a) of the render decode's division-free quotients against
+    IEEE division, over every 0 < a < b <= b_max (single frames: every span up to 255), and of the ray
+    sampler's axis weights (vbt_selftest_key_division in vbt_b200.h)."""
     r = (C.c_uint64 * 2)()
     _check(_lib.vbt_selftest_key_division(b_max, r, device))
     return int(r[0]), int(r[1])

@@ -683,6 +683,7 @@ int vbt_selftest_key_division(uint32_t b_max, uint64_t* result, int device)
     cudaError_t e = cudaMemcpy(d, init, sizeof(init), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) {
         launch_key_division_check(b_max, d, nullptr);
+        launch_span_check(d, nullptr);
         e = cudaGetLastError();
     }
     unsigned long long h[2] = {0ull, 0ull};

@@ -1273,8 +1273,9 @@ void release_mixed_graph(MixedStepGraph& g)
 }
 
 // Exhaustive check of div_small_rn (the render decode's interval quotient) against IEEE division:
-// every pair 0 < a < b <= b_max, with RN(1/b) as the decode forms it.  Counts mismatches and keeps
-// the smallest failing (b << 16 | a).
+// every pair 0 < a < b <= b_max, with RN(1/b) as the decode forms it; and of div_u8_rn (the quotient of
+// single frames) for every 0 <= a <= b <= 255.  Counts mismatches and keeps the smallest failing
+// (b << 16 | a).
 __global__ void key_division_check_kernel(uint32_t b_max, unsigned long long* bad, unsigned long long* first)
 {
     unsigned long long local = 0;
@@ -1284,6 +1285,14 @@ __global__ void key_division_check_kernel(uint32_t b_max, unsigned long long* ba
         for (uint32_t a = 1u + threadIdx.x; a < b; a += blockDim.x) {
             const float q = div_small_rn((float)a, bf, y);
             if (__float_as_uint(q) != __float_as_uint(__fdiv_rn((float)a, bf))) {
+                ++local;
+                atomicMin(first, ((unsigned long long)b << 16) | a);
+            }
+        }
+    }
+    for (uint32_t b = 1u + blockIdx.x; b <= 255u; b += gridDim.x) {
+        for (uint32_t a = threadIdx.x; a <= b; a += blockDim.x) {
+            if (__float_as_uint(div_u8_rn((float)a, (float)b)) != __float_as_uint(__fdiv_rn((float)a, (float)b))) {
                 ++local;
                 atomicMin(first, ((unsigned long long)b << 16) | a);
             }

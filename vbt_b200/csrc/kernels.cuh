@@ -126,6 +126,7 @@ void launch_control_cache(const DeviceAsset& a, const int* frames, int nframes, 
 void launch_render_window_oracle(const DeviceAsset& a, int t0, int n, const float* vals, uint64_t frame_stride,
                                  unsigned long long* stats, cudaStream_t s);
 void launch_key_division_check(uint32_t b_max, unsigned long long* d_out, cudaStream_t s);
+void launch_span_check(unsigned long long* d_out, cudaStream_t s);   // the ray sampler's axis weights (sample.cu)
 void launch_sci_window_oracle(const DeviceAsset& a, int t0, int n, const float* vals, uint64_t frame_stride,
                               unsigned long long* stats, cudaStream_t s);
 // Plain path: one CTA per leaf of the whole leaf grid, one frame per launch (the reference

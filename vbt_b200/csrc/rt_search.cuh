@@ -214,7 +214,7 @@ __device__ __forceinline__ KeyWindow key_start(const LeafStream& s, uint32_t des
 // a / b for 0 <= a <= b <= 255, correctly rounded: the product with the approximate reciprocal and one
 // fused remainder step (P. Markstein, IBM J. Res. Dev. 34(1), 1990).  A quotient of such integers is at
 // least 2^-9 of a unit in the last place away from a rounding boundary, far more than the reciprocal's
-// error moves the corrected one (checked for every pair with reciprocals off by up to two units).
+// error moves the corrected one.  vbt_selftest_key_division checks every pair.
 __device__ __forceinline__ float div_u8_rn(float a, float b)
 {
     float y;

@@ -142,7 +142,7 @@ constexpr float span_start(uint32_t j)
 // locate_coord for a compile-time resolution R (4 or 6) and a position from +0 on that is 0 or not
 // below 2^-63.  The quotient (c - c0) / span is div_small_rn's: a fused remainder after the product
 // with RN(1 / span), equal to IEEE division for every significand of the numerator and every span of
-// these grids (checked exhaustively on the host).
+// these grids.  vbt_selftest_key_division checks every position.
 template <uint32_t R>
 __device__ __forceinline__ uint32_t locate_span(const float4* __restrict__ spans, float pos, float top, float& w)
 {
@@ -153,6 +153,35 @@ __device__ __forceinline__ uint32_t locate_span(const float4* __restrict__ spans
     const float4 s = spans[(R == 4u ? 0u : 3u) + i];
     w = div_small_rn(__fsub_rn(c, s.x), s.y, s.z);
     return i;
+}
+
+// locate_span against locate_coord for every position it takes and every extent: mismatches in out[0], the smallest
+// failing 2^63 | R << 40 | extent << 32 | position bits in out[1].
+template <uint32_t R>
+__device__ __forceinline__ void span_check(const float4* spans, uint32_t bits, unsigned long long* out)
+{
+    const float pos = __uint_as_float(bits);
+    for (uint32_t ext = 1u; ext <= 8u; ++ext) {
+        uint32_t i0, i1;
+        float want, got;
+        locate_coord(pos, ext, R, i0, i1, want);
+        const uint32_t i = locate_span<R>(spans, pos, (float)(ext - 1u), got);
+        if (i != i0 || i + 1u != i1 || __float_as_uint(got) != __float_as_uint(want)) {
+            atomicAdd(out, 1ull);
+            atomicMin(out + 1, (1ull << 63) | ((unsigned long long)R << 40) | ((unsigned long long)ext << 32) | bits);
+        }
+    }
+}
+__global__ void __launch_bounds__(256) span_check_kernel(unsigned long long* out)
+{
+    __shared__ float4 s_spans[kSpanRows];
+    fill_spans(s_spans);
+    const uint32_t first = 0x20000000u, past = 0x41000000u;   // 2^-63 to 8
+    for (uint32_t b = first - 1u + blockIdx.x * blockDim.x + threadIdx.x; b < past; b += gridDim.x * blockDim.x) {
+        const uint32_t bits = b < first ? 0u : b;
+        span_check<4u>(s_spans, bits, out);
+        span_check<6u>(s_spans, bits, out);
+    }
 }
 
 // sample_stream over a cached grid of compile-time resolution: the same lerps on the same controls.
@@ -656,6 +685,8 @@ __global__ void __launch_bounds__(128) smoke_sample_kernel(DeviceAsset a, vbt_sa
 }
 
 }  // namespace
+
+void launch_span_check(unsigned long long* d_out, cudaStream_t s) { span_check_kernel<<<1184, 256, 0, s>>>(d_out); }
 }  // namespace vbtb
 
 using namespace vbtb;
