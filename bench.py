@@ -100,62 +100,48 @@ def algorithmic_bytes_per_frame(rows):
 
 
 class ClockSampler:
-    FIELDS = ("clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.hw_slowdown,"
-              "clocks_event_reasons.hw_thermal_slowdown,clocks_event_reasons.sw_thermal_slowdown,"
-              "clocks_event_reasons.sw_power_cap")
+    """SM clock and slowdown reasons during the timed region, read through NVML every 2 ms (a timed region of 20
+    steps is 10 ms; nvidia-smi takes a sample every 50 ms at best)."""
+
+    REASONS = {"hw_slowdown": 0x8, "hw_thermal_slowdown": 0x40, "sw_thermal_slowdown": 0x20, "sw_power_cap": 0x4}
 
     def __init__(self, index):
         self.index = index
-        self.proc = None
-        self.lines = []
+        self.thread = None
+        self.samples = []
 
     def start(self):
-        """nvidia-smi every 50 ms; each line is stamped with the host clock when it arrives."""
         try:
-            self.proc = subprocess.Popen(["nvidia-smi", "-i", str(self.index), f"--query-gpu={self.FIELDS}",
-                                          "--format=csv,noheader,nounits", "-lms", "50"], stdout=subprocess.PIPE,
-                                         stderr=subprocess.DEVNULL, text=True, bufsize=1)
+            import pynvml
+            pynvml.nvmlInit()
+            dev = pynvml.nvmlDeviceGetHandleByIndex(self.index)
+            self.max_mhz = float(pynvml.nvmlDeviceGetMaxClockInfo(dev, pynvml.NVML_CLOCK_SM))
         except Exception:
-            self.proc = None
             return
+        self.running = True
 
         def reader():
-            for line in self.proc.stdout:
-                self.lines.append((time.time(), line))
+            while self.running:
+                try:
+                    self.samples.append((time.time(), float(pynvml.nvmlDeviceGetClockInfo(dev, pynvml.NVML_CLOCK_SM)),
+                                         int(pynvml.nvmlDeviceGetCurrentClocksThrottleReasons(dev))))
+                except pynvml.NVMLError:
+                    return
+                time.sleep(0.002)
 
         self.thread = threading.Thread(target=reader, daemon=True)
         self.thread.start()
-        t0 = time.time()
-        while not self.lines and time.time() - t0 < 10.0:   # nvidia-smi takes a moment to start
-            time.sleep(0.05)
 
     def stop(self, t0, t1):
-        """Samples that arrived inside the host-clock window [t0, t1] of the timed region."""
-        if self.proc is None:
-            return {"sm_mhz": None, "sm_max_mhz": None, "samples": 0, "reasons": ["nvidia-smi unavailable"]}
-        self.proc.terminate()
-        try:
-            self.proc.wait(timeout=5)
-        except Exception:
-            self.proc.kill()
-        sm, mx, reasons = [], [], set()
-        names = ["hw_slowdown", "hw_thermal_slowdown", "sw_thermal_slowdown", "sw_power_cap"]
-        for ts, line in list(self.lines):
-            if ts < t0 or ts > t1:
-                continue
-            parts = [p.strip() for p in line.split(",")]
-            if len(parts) < 7:
-                continue
-            try:
-                sm.append(float(parts[0]))
-                mx.append(float(parts[1]))
-            except ValueError:
-                continue
-            for n, v in zip(names, parts[3:7]):
-                if v.lower() == "active":
-                    reasons.add(n)
-        return {"sm_mhz": statistics.median(sm) if sm else None, "sm_max_mhz": max(mx) if mx else None,
-                "samples": len(sm), "reasons": sorted(reasons)}
+        """Samples taken inside the host-clock window [t0, t1] of the timed region."""
+        if self.thread is None:
+            return {"sm_mhz": None, "sm_max_mhz": None, "samples": 0, "reasons": ["NVML unavailable"]}
+        self.running = False
+        self.thread.join(timeout=5)
+        inside = [s for s in self.samples if t0 <= s[0] <= t1]
+        reasons = sorted(n for n, bit in self.REASONS.items() if any(s[2] & bit for s in inside))
+        return {"sm_mhz": statistics.median(s[1] for s in inside) if inside else None, "sm_max_mhz": self.max_mhz,
+                "samples": len(inside), "reasons": reasons}
 
 
 def measured_peak():
