@@ -370,14 +370,14 @@ int vbt_selftest_key_division(uint32_t b_max, uint64_t* result, int device);
 /* ---- Batched timeline: autotuned, graph-captured ---------------------------------------------
  * No counterpart in the reference.  The current-frame cache of a frame range is a page-table build
  * plus one decode launch per `frames_per_launch` frames.  The launch shape (leaf per CTA: the
- * TMA-staged kernel; leaf per warp: eight leaves per CTA), the frames per launch and the grid are
+ * TMA-staged kernel; leaf per warp: four leaves per CTA), the frames per launch and the grid are
  * chosen per asset by timing the candidates on the caller's output (vbt_autotune_cache), or set
  * directly (vbt_set_tuning).  vbt_decode_cache_timeline then runs the whole range; with use_graph
  * it is captured once into a CUDA graph per (first frame, count, output, stride) and replayed with
  * one cudaGraphLaunch.  Output as vbt_decode_cache: d_out[f * frame_stride + rank * 512 + voxel]. */
 typedef struct {
     uint32_t variant;            /* 0: leaf per CTA; 1: leaf per warp */
-    uint32_t frames_per_launch;  /* 1 .. 64 */
+    uint32_t frames_per_launch;  /* 1 .. 128 */
     int grid;                    /* CTAs per launch, 0 = one wave */
     float ms_per_frame;          /* measured by vbt_autotune_cache (0 when set by hand) */
     float ms_per_frame_default;  /* the untuned configuration (leaf per CTA, 48 frames, one wave) */

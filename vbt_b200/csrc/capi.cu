@@ -612,18 +612,13 @@ int vbt_decode_frames_host(vbt_asset* a, const int* frames, int nframes, float* 
 int vbt_decode_window(vbt_asset* a, int t0, int n, float* d_out, uint64_t frame_stride, void* stream)
 {
     if (!a || !d_out) return fail(VBT_STATUS_INVALID_ARGUMENT, "null argument");
-    if (a->hdr.profile_type == 2u) {
-        if (n < 1 || n > 64 || t0 < 0 || (uint64_t)t0 + (uint64_t)n > a->hdr.frames)
-            return fail(VBT_STATUS_INVALID_ARGUMENT, "window must be 1..64 frames inside [0, frames)");
-        if (frame_stride < 512ull * a->hdr.leaf_count)
-            return fail(VBT_STATUS_INVALID_ARGUMENT, "frame_stride below leaf_count * 512");
-        DeviceGuard guard(a->device);
-        launch_sci_window(a->dev, t0, n, d_out, frame_stride, static_cast<cudaStream_t>(stream));
-        return check_launch("sci_frames_kernel");
-    }
+    const bool sci = a->hdr.profile_type == 2u;
     if (n < 1 || n > 64 || t0 < 0 || (uint64_t)t0 + (uint64_t)n > a->hdr.frames)
-        return fail(VBT_STATUS_INVALID_ARGUMENT, "render windows must cover 1..64 frames inside [0, frames)");
-    if ((reinterpret_cast<uintptr_t>(d_out) & 15u) != 0u || (frame_stride & 3u) != 0u)
+        return fail(VBT_STATUS_INVALID_ARGUMENT, sci ? "window must be 1..64 frames inside [0, frames)"
+                                                     : "render windows must cover 1..64 frames inside [0, frames)");
+    if (sci && frame_stride < 512ull * a->hdr.leaf_count)
+        return fail(VBT_STATUS_INVALID_ARGUMENT, "frame_stride below leaf_count * 512");
+    if (!sci && ((reinterpret_cast<uintptr_t>(d_out) & 15u) != 0u || (frame_stride & 3u) != 0u))
         return fail(VBT_STATUS_INVALID_ARGUMENT, "output must be 16-byte aligned, frame_stride a multiple of 4");
     DeviceGuard guard(a->device);
     int frames[64];

@@ -1311,6 +1311,6 @@ void launch_key_division_check(uint32_t b_max, unsigned long long* d_out, cudaSt
 
 }  // namespace vbtb
 
-// (d) windows and their error oracles
-#include "sci_window.cuh"
-#include "render_window.cuh"
+// (d) the error oracles of windows
+#include "sci_window_oracle.cuh"
+#include "render_window_oracle.cuh"

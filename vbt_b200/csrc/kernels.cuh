@@ -63,8 +63,6 @@ constexpr uint32_t kLeafFixedBytes =
 constexpr int kWalkThreads = 256;
 constexpr int kWalkTile = 256;   // leaves per walker CTA (one scan element per thread)
 
-// Decode work is done one leaf per warp; kDecodeWarps warps per CTA.
-constexpr int kDecodeWarps = 8;
 constexpr int kCtrlSlots = 343 + 512;   // coarse (<= 7^3) + fine (<= 7^3) or shell (<= 512) values
 // per-warp shared slots: max(render controls, scientific 64 controls + 16 basis grids of 4^3)
 constexpr int kWarpSlots = 64 + 16 * 64 > kCtrlSlots ? 64 + 16 * 64 : kCtrlSlots;
@@ -117,8 +115,6 @@ void launch_decode_dense(const DeviceAsset& a, uint32_t seq, const int* frames, 
 void launch_decode_cache_warp(const DeviceAsset& a, const int* frames, int nframes, float* out, uint64_t stride,
                               int grid, cudaStream_t s);
 int decode_warp_grid();
-// (d) scientific window decode, frames [t0, t0 + n), n <= 64, cache layout (the exact frames kernel).
-void launch_sci_window(const DeviceAsset& a, int t0, int n, float* out, uint64_t frame_stride, cudaStream_t s);
 // FP64 oracle of a scientific window: stats[0] max |err| (double bits), stats[1] sum err^2
 // (double), stats[2] / stats[3] oracle min / max (order-preserving bits).
 void launch_control_cache(const DeviceAsset& a, const int* frames, int nframes, float* out, uint64_t stride,
@@ -133,7 +129,8 @@ void launch_sci_window_oracle(const DeviceAsset& a, int t0, int n, const float* 
 // Studio dispatch shape, VBTStudio/frontend/src/volume_renderer.cpp:704-735).
 void launch_decode_cache_plain(const DeviceAsset& a, int frame, float* out, cudaStream_t s);
 // Point queries: q[4*i..] = (x, y, z, t); out[i].
-// sparse: most leaves are EMPTY (the compacting kernel), else one thread per query
+// sparse: most leaves are EMPTY (a warp answers the queries that need no decoding on its way through 256 of them
+// and decodes the others in full batches), else each warp decodes 32
 void launch_query_points(const DeviceAsset& a, const uint32_t* q, uint64_t n, float* out, bool sparse, cudaStream_t s);
 // Point queries of k requests over several assets in one launch (a device array of DeviceAsset).
 // seg: starts[0..k] (first query of each request, starts[k] = n), asset[k], then 8-byte aligned

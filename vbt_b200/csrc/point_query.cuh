@@ -10,10 +10,9 @@
 // forms its own query's lerps from the corner values, in the reference's order.  No step repeats
 // another's work, and a batch of a few queries is still only one chain long.
 // Bound by instruction issue (67 % of the slots, 63 warp instructions per query on a scientific
-// field), then by L1/L2 latency; DRAM is idle.  Measured on a B200 against one thread per query:
-// 1,000,000 random queries of a 256^3 x 96 plume 138 -> 62 us, of a dense 128^3 x 40 fire 355 -> 152,
-// of a 128^3 x 64 scientific field 203 -> 89; 1,000 queries 34 -> 9 (the call; 35 -> 5 on the device).
-// Eight lanes per query from start to end, the shape between the two, gave 79, 226 and 165.
+// field), then by L1/L2 latency; DRAM is idle.  On a B200: 1,000,000 random queries of a 256^3 x 96 plume
+// 57 us, of a dense 128 x 128 x 192 x 40 fire 147, of a 128^3 x 64 scientific field 86; 1,000 queries 6.7 (one
+// thread per query 138, 355, 203 and 34; eight lanes to a query from start to end 79, 226, 165).
 #pragma once
 
 namespace vbtb {

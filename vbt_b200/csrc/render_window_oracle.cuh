@@ -1,12 +1,6 @@
-// render_window.cuh -- the FP64 error oracle of render-temporal windows.  Included by kernels.cu after
-// sci_window.cuh.
-//
-// A window is a run of frames of the cache, and its decode is the cache's (launch_decode_cache): with the
-// key cursors carried through all frames a frame costs less than splitting the voxels at the union of the
-// controls' key frames into three BF16 terms for a contraction with hat functions (24 tcgen05.mma per leaf
-// and 16 frames), which also decodes every frame whose neighbours hold keys.  B200, contraction against
-// cache: 64 frames of a 128 x 100 x 90 fire 645 / 221 us, of a 120 x 100 x 110 plume 254 / 80, 16 frames
-// of a 72 x 106 x 49 fire 77 / 36, one frame of the first 97 / 16.
+// render_window_oracle.cuh -- the FP64 error oracle of render-temporal windows.  Included by kernels.cu after
+// sci_window_oracle.cuh.  A window is a run of frames of the cache, and its decode is the cache's
+// (launch_decode_cache).
 #pragma once
 
 namespace vbtb {

@@ -14,8 +14,8 @@
 //    a (1 - t)), which makes the control rows of every lane the same register names;
 //  - events: the keys of a time bin are read once per bin, and the events of a frame go through a
 //    shared-memory row of residuals that the z step adds; frames without events skip it.
-// 64 frames of a 128^3 field (537 MB written, 83 us at the measured copy rate) on a B200: 1,388 us with
-// one warp per leaf in the per-voxel form, 175 us so.  Bound by instruction issue (about 400 warp
+// 64 frames of a 128^3 field (537 MB written, 83 us at the measured copy rate) on a B200: cache 162 us, dense
+// frames 175 (voxel by voxel 1,203 and 1,388).  Bound by instruction issue (about 400 warp
 // instructions per leaf and frame over all leaf kinds, 55 % of the slots) beside the stores.
 #pragma once
 
@@ -227,7 +227,7 @@ __device__ __forceinline__ bool sci_common_shape(const AssetGeom& g, const LeafE
 // and frame by frame 1,221, 1,467 and 4,348).  An instantiation of its own, since its controls and sums cost
 // the other kernel registers.
 // Four CTAs of 128 registers: with 96 registers and five, the spills and the wider spread of the writes
-// cost more than the warps hide (222 against 265 us).
+// cost more than the warps hide (an earlier form of the loop: 265 us against 222).
 // LOOSE: a cache that starts at any float, its frames any number of floats apart (an instantiation of its
 // own: the test in the one kernel costs an aligned window of 64 frames of 128^3 1.5 %).
 template <bool DENSE, bool LOOSE, bool WIDE>
@@ -545,8 +545,8 @@ __global__ void __launch_bounds__(kSciWarps * 32, 4) sci_frames_kernel(DeviceAss
 }
 
 // Frames per item: 16 where that leaves twelve or more items for every resident warp, else 8, and 4
-// where those would not give each warp two (an item's set-up costs about three frames; 64 frames of
-// 128^3: 8 frames per item 216 us, 16 235; of 256 x 128 x 128: 385 and 375).
+// where those would not give each warp two (an item's set-up costs about three frames; an earlier form of the
+// loop, 64 frames of 128^3: 8 frames per item 216 us, 16 235; of 256 x 128 x 128: 385 and 375).
 template <bool DENSE, bool LOOSE, bool WIDE>
 static void launch_sci_variant(const DeviceAsset& a, const FrameList& fl, float* out, uint64_t stride, int grid,
                                cudaStream_t s)

@@ -1,11 +1,6 @@
-// sci_window.cuh -- the FP64 error oracle of scientific windows and the window launcher.  Included by
-// kernels.cu (it uses that file's scientific helpers).
-//
-// A scientific window is decoded by the exact frames kernel (sci_frames.cuh): with a leaf's
-// coefficients, weights and events in registers a frame costs less on the CUDA cores than splitting
-// its controls into three BF16 terms, 48 MMAs per leaf-window and an epilogue that adds corners and
-// events -- 64 frames of a 128^3 field on a B200: 162 us against 499 us for the contraction -- and the
-// values are the exact path's own.
+// sci_window_oracle.cuh -- the FP64 error oracle of scientific windows (and of any cache of scientific frames).
+// Included by kernels.cu (it uses that file's scientific helpers).  The windows themselves are decoded by the
+// frames kernel (sci_frames.cuh).
 #pragma once
 
 namespace vbtb {
@@ -151,16 +146,6 @@ __global__ void __launch_bounds__(256) sci_window_oracle_kernel(DeviceAsset a, i
         atomicMin(stats + 2, lo);
         atomicMax(stats + 3, hi);
     }
-}
-
-// Frames [t0, t0 + n), n <= 64, of every leaf (all leaves of a scientific asset are in its page table,
-// in order): out[f * frame_stride + leaf * 512 + voxel].
-void launch_sci_window(const DeviceAsset& a, int t0, int n, float* out, uint64_t frame_stride, cudaStream_t s)
-{
-    FrameList fl{};
-    fl.n = n;
-    for (int i = 0; i < n; ++i) fl.f[i] = t0 + i;
-    launch_sci_frames<false>(a, fl, out, frame_stride, 0, s);
 }
 
 void launch_sci_window_oracle(const DeviceAsset& a, int t0, int n, const float* vals, uint64_t frame_stride,

@@ -4,7 +4,7 @@
 // A timeline is a page-table build followed by ceil(n / frames_per_launch) cache-decode launches.
 // The autotuner times every candidate shape on the caller's own output buffer with CUDA events
 // and keeps the fastest: leaf per CTA (the TMA-staged kernel; 16, 24, 32, 48, 64, 96 or 128
-// frames per launch) or leaf per warp (8 leaves per CTA; 16, 32 or 64 frames, one or two waves).  All shapes
+// frames per launch) or leaf per warp (4 leaves per CTA; 16, 32 or 64 frames, one or two waves).  All shapes
 // write identical values.
 #include <cuda_runtime.h>
 
