@@ -11,15 +11,15 @@
 // another's work, and a batch of a few queries is still only one chain long.
 // Bound by instruction issue (67 % of the slots, 63 warp instructions per query on a scientific
 // field), then by L1/L2 latency; DRAM is idle.  On a B200: 1,000,000 random queries of a 256^3 x 96 plume
-// 57 us, of a dense 128 x 128 x 192 x 40 fire 147, of a 128^3 x 64 scientific field 86; 1,000 queries 6.7 (one
+// 50 us, of a dense 128 x 128 x 192 x 40 fire 133, of a 128^3 x 64 scientific field 83; 1,000 queries 6.2 (one
 // thread per query 138, 355, 203 and 34; eight lanes to a query from start to end 79, 226, 165).
 #pragma once
 
 namespace vbtb {
 
-// Eight CTAs per SM: 64 registers (some set-up values spill) and 32 warps, which hide the reads better
-// than 24 warps at 80 registers (fire 175 us); 40 warps at 48 gain on the fire (143) and lose on the
-// plume (74).
+// Eight CTAs per SM: at most 64 registers (the kernels with scientific queries spill some set-up values) and 32
+// warps, which hide the reads better than 24 warps at 80 registers (fire 175 us against 153 in the kernel for
+// both kinds; 40 warps at 48 registers 143, but the plume 74 against 66).
 // Events of a batch that eight lanes each look up in turn; more go to their own lanes.
 constexpr int kPqEvents = 8;
 constexpr int kPqWarps = 4, kPqCtas = 8, kPqThreads = 32 * kPqWarps, kPqBatch = 32;
@@ -243,6 +243,11 @@ __device__ __forceinline__ uint32_t corner_step(uint32_t k, uint32_t res)
     return res < 2u ? 0u : (k & 1u) + ((k >> 1) & 1u) * res + (k >> 2) * res * res;
 }
 
+// The queries of a launch: of render files, of scientific files, or of both (a serving step).  A kernel for one
+// kind has no registers spilled for the other: against the kernel for both, 1,000,000 queries of the plume 57 -> 50
+// us, of the field 86 -> 83, a thousand 6.8 -> 6.2.
+enum : int { kRenderOnly, kSciOnly, kBoth };
+
 // Up to 32 queries, one per lane (`on`): value and where to put it are the lane's own.
 template <class Resolve>
 __device__ __forceinline__ void query_batch(QueryShared& sh, const float2* table, uint32_t batch, bool on, uint64_t i,
@@ -254,6 +259,8 @@ __device__ __forceinline__ void query_batch(QueryShared& sh, const float2* table
     bool second = false, event = false, alone = false, tbasis = false;
     const auto r = resolve.request(on ? i : 0);
     const DeviceAsset& a = resolve.asset(r);
+    constexpr bool kRt = Resolve::kFamily != kSciOnly, kSc = Resolve::kFamily != kRenderOnly;   // kinds that occur
+    const bool sci = !kRt || (kSc && a.g.profile == 2u);
     // 1. the lane's query
     if (on) {
         const uint4 qq = q[i];
@@ -269,7 +276,7 @@ __device__ __forceinline__ void query_batch(QueryShared& sh, const float2* table
         c.lw = a.payload + e.word_off;
         if (st != kOk) {
             record_error(resolve.err(r), leaf, st);
-        } else if (a.g.profile == 2u) {
+        } else if (sci) {
             lx = qq.x & 7u, ly = qq.y & 7u, lz = qq.z & 7u;
             if (t >= a.g.frames) {   // the reference indexes its per-frame tables out of range here
                 record_error(resolve.err(r), leaf, kErrDecodeOob);
@@ -337,8 +344,7 @@ __device__ __forceinline__ void query_batch(QueryShared& sh, const float2* table
     const bool residual = tbasis || (event && !alone);
     const uint32_t m3 = __ballot_sync(0xFFFFFFFFu, residual);
     const uint32_t below = (1u << lane) - 1u;
-    const bool sci = a.g.profile == 2u;
-    const uint32_t msci = __ballot_sync(0xFFFFFFFFu, on && sci);
+    const uint32_t msci = !kRt ? 0xFFFFFFFFu : !kSc ? 0u : __ballot_sync(0xFFFFFFFFu, on && sci);
     if (second) sh.second[__popc(m2 & below)] = (uint8_t)lane;
     if (residual) sh.residuals[__popc(m3 & below)] = (uint8_t)lane;
     __syncwarp();
@@ -361,7 +367,7 @@ __device__ __forceinline__ void query_batch(QueryShared& sh, const float2* table
         }
         sh.val[s * 17u + sub] = v;
     }
-    const uint32_t n2 = (uint32_t)__popc(m2), n3 = (uint32_t)__popc(m3);
+    const uint32_t n2 = (uint32_t)__popc(m2), n3 = kSc ? (uint32_t)__popc(m3) : 0u;
     for (uint32_t k = group; k < n2; k += 4u) {
         const uint32_t s = sh.second[k];
         const QueryCell& c = sh.cell[s];
@@ -398,7 +404,7 @@ __device__ __forceinline__ void query_batch(QueryShared& sh, const float2* table
         const float* v = sh.val + lane * 17u;
         const uint32_t lx = place & 7u, ly = (place >> 3) & 7u, lz = place >> 6;
         float out = 0.0f;
-        if (kind == kRender) {
+        if (kRt && kind == kRender) {
             const LeafEntry e = a.entries[leaf];   // again, so that it holds no registers meanwhile
             const uint32_t cres = (e.header >> 6) & 7u, fres = (e.header >> 9) & 7u;
             out = cell_value(table, render_grid(cres), cres, lx, ly, lz, v);
@@ -421,7 +427,7 @@ __device__ __forceinline__ void query_batch(QueryShared& sh, const float2* table
                                                 (e.info & kFlagSorted) != 0u));
             }
             if ((e.info & kFlagOccClamp) && !in_occ && out < 0.0f) out = 0.0f;
-        } else if (kind == kSci) {
+        } else if (kSc && kind == kSci) {
             const float coarse = cell_value(table, 2, 4u, lx, ly, lz, v);
             float res = residual ? v[16] : 0.0f;
             if (event && alone) {
@@ -432,7 +438,7 @@ __device__ __forceinline__ void query_batch(QueryShared& sh, const float2* table
             if (second) res = (sh.cell[lane].kf & 3u) == 2u ? cell_value(table, 3, 3u, lx, ly, lz, v + 8)
                                                     : cell_value(table, 2, 4u, lx, ly, lz, v + 8);
             out = __fadd_rn(coarse, res);
-        } else if (kind == kSciGeneral) {
+        } else if (kSc && kind == kSciGeneral) {
             bool oob = false;
             out = sci_point_general(a, a.entries[leaf], lx, ly, lz, sh.cell[lane].t, &oob);
             if (oob) record_error(resolve.err(r), leaf, kErrDecodeOob);
@@ -531,7 +537,9 @@ static unsigned query_blocks(uint64_t n, uint32_t chunk)
     return (unsigned)((n + per - 1) / per);
 }
 
+template <int FAMILY>
 struct OneAssetQueries {
+    static constexpr int kFamily = FAMILY;
     const DeviceAsset& a;
     float* __restrict__ out;
     __device__ __forceinline__ bool sparse(uint64_t) const { return a.g.sparse != 0u; }
@@ -541,11 +549,12 @@ struct OneAssetQueries {
     __device__ __forceinline__ void put(int, uint64_t i, float v) const { out[i] = v; }
 };
 
+template <int FAMILY>
 __global__ void __launch_bounds__(kPqThreads, kPqCtas) query_points_kernel(const __grid_constant__ DeviceAsset a,
                                                                   const uint4* __restrict__ q, uint64_t n,
                                                                   uint32_t chunk, float* __restrict__ out)
 {
-    query_chunk(n, chunk, q, OneAssetQueries{a, out});
+    query_chunk(n, chunk, q, OneAssetQueries<FAMILY>{a, out});
 }
 
 // Point queries of several requests over several resident assets in one launch.  The segment
@@ -553,6 +562,7 @@ __global__ void __launch_bounds__(kPqThreads, kPqCtas) query_points_kernel(const
 // assets[asset[r]]) and, 8-byte aligned after them, outs[k] (request r's result array).  Request
 // r's decode errors go to errs[r].
 struct BatchQueries {
+    static constexpr int kFamily = kBoth;
     const DeviceAsset* __restrict__ assets;
     const uint32_t* __restrict__ seg;
     uint32_t k;
@@ -598,7 +608,8 @@ void launch_query_points(const DeviceAsset& a, const uint32_t* q, uint64_t n, fl
 {
     if (n == 0) return;
     const uint32_t chunk = query_chunk_size(n, sparse ? kPqSparseChunk : kPqDenseChunk);
-    query_points_kernel<<<query_blocks(n, chunk), kPqThreads, 0, s>>>(a, reinterpret_cast<const uint4*>(q), n, chunk, out);
+    const auto kernel = a.g.profile == 2u ? query_points_kernel<kSciOnly> : query_points_kernel<kRenderOnly>;
+    kernel<<<query_blocks(n, chunk), kPqThreads, 0, s>>>(a, reinterpret_cast<const uint4*>(q), n, chunk, out);
 }
 
 }  // namespace vbtb
