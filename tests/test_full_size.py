@@ -10,7 +10,7 @@ to the host, where the oracle (oracle/vbt_oracle.c) loads it from memory.
             signs of phi;
   config 3, the fire's density (EMPTY leaves outside the growing sphere) and temperature (the
             largest of the three fields: noise in every leaf), 384 x 384 x 512 x 120: the page
-            table, the cache of three frames bit for bit, and a 16-frame tensor-core window within
+            table, the cache of three frames bit for bit, and a 16-frame window within
             1e-6 of the field's range of the FP64 oracle.
 """
 import os

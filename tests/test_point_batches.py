@@ -37,7 +37,7 @@ def test_batch_edges(name, vbt, cuda, oracle):
         a.sync_status()
         got, want = out.cpu().numpy(), f.query(q)
         assert got[n] == -7.0, (name, n)
-        if sci:   # the reference's double sum against a compensated one: one rounding of the field's range
+        if sci:   # one rounding of the field's range (bit for bit in test_sci_kinds.py)
             assert np.abs(got[:n].astype(np.float64) - want).max() <= 1e-6 * scale, (name, n)
         else:
             assert np.array_equal(got[:n].view(np.uint32), want.view(np.uint32)), (name, n)

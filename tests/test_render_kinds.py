@@ -1,6 +1,6 @@
 """Render-temporal leaves of every grid resolution, of FP32 keys, with fine grids and Mode2 shells -- files whose
 leaves are mostly of the common shape (FP16 keys, 4^3 grids, 6^3 fine grids) and files whose leaves are not --
-as caches and dense frames of frame counts on both sides of the rules for few frames, slices and point queries,
+as caches, windows and dense frames of frame counts on both sides of the rules for few frames, slices and point queries,
 against the oracle bit for bit."""
 import numpy as np
 import pytest
@@ -45,6 +45,10 @@ def test_kinds(name, dims, vbt, cuda, oracle):
             dense = cuda.full((n, Z, Y, X), -7.0, device="cuda")
             a.decode_frames(frames, dense)
             same(dense, want[frames], "dense", frames)
+    for t0, n in ((0, 2), (3, 20), (1, 32)):
+        out = cuda.full((n, a.active_count, 512), -7.0, device="cuda")
+        a.decode_window(t0, n, out, frame_stride=out.stride(0))
+        same(out, cache[t0:t0 + n], "window", t0, n)
     for z in range(Z):
         rows = cuda.full((5, Y, X), -7.0, device="cuda")
         a.query_slice(z, 14, 19, rows)

@@ -1,9 +1,8 @@
-"""(d) Window decode of scientific leaves on the tensor cores (vbt_decode_window) and its FP64
-error oracle (vbt_window_error).
+"""(d) Window decode (vbt_decode_window) and its FP64 error oracle (vbt_window_error).
 
-The window path is not bit-exact by design (split-BF16 products, FP32 accumulation); the bar is
-1e-6 of the field range against the FP64 oracle and against the exact per-frame decode.  The
-oracle is checked to report a planted deviation of known size.
+Windows are decoded by the cache's kernels; the bar here is 1e-6 of the field range against the FP64 oracle
+and against the per-frame decode (bit for bit in test_sci_kinds.py and test_render_kinds.py).  The oracle is
+checked to report a planted deviation of known size.
 """
 import os
 
@@ -96,7 +95,7 @@ def test_window_rejects_long_windows(vbt, cuda):
     s.close()
 
 
-# ---- render-temporal windows: exact voxels at the knots, hat-basis contraction on the tensor cores
+# ---- render-temporal windows
 
 
 def render_paths():
